@@ -37,10 +37,46 @@ __host__ __device__ __forceinline__ double2 mk(double x, double y) { return make
 __host__ __device__ __forceinline__ float2 mk(float x, float y) { return make_float2(x, y); }
 __device__ __forceinline__ double2 operator+(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 operator-(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ float2 operator+(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 operator-(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// FP32 complex sums, differences and products with a real number use the packed
+// f32x2 instructions: both components in one issue slot, each rounded as the
+// scalar instruction rounds it.  The register FFTs are mostly such operations
+// (a 30-point one: 242 instructions instead of 396); products with a twiddle
+// stay scalar, because a packed form needs as many moves as it saves.  B = 15,
+// 32^3, FP32: plane pass 1.96 -> 1.84 ms, omega planes 0.210 -> 0.191,
+// synthesis 2.84 -> 2.78.
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ float2 operator+(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a.x, a.y)), "l"(pack2(b.x, b.y)));
+  return unpack2(r);
+}
+__device__ __forceinline__ float2 operator-(float2 a, float2 b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a.x, a.y)), "l"(pack2(b.x, b.y)));
+  return unpack2(r);
+}
 __device__ __forceinline__ double2 operator*(double s, double2 a) { return make_double2(s * a.x, s * a.y); }
-__device__ __forceinline__ float2 operator*(float s, float2 a) { return make_float2(s * a.x, s * a.y); }
+__device__ __forceinline__ float2 operator*(float s, float2 a) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(s, s)), "l"(pack2(a.x, a.y)));
+  return unpack2(r);
+}
+// a + s b, s real
+__device__ __forceinline__ double2 rfma(double s, double2 b, double2 a) { return make_double2(fma(s, b.x, a.x), fma(s, b.y, a.y)); }
+__device__ __forceinline__ float2 rfma(float s, float2 b, float2 a) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pack2(s, s)), "l"(pack2(b.x, b.y)), "l"(pack2(a.x, a.y)));
+  return unpack2(r);
+}
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
 }
@@ -53,6 +89,13 @@ __device__ __forceinline__ double2 cfma(double2 b, double2 c, double2 a) {
 }
 __device__ __forceinline__ float2 cfma(float2 b, float2 c, float2 a) {
   return make_float2(fmaf(b.x, c.x, fmaf(-b.y, c.y, a.x)), fmaf(b.x, c.y, fmaf(b.y, c.x, a.y)));
+}
+// a + i b (NEG: a - i b)
+template <bool NEG, typename C> __device__ __forceinline__ C cadd_i(C a, C b) {
+  C r;
+  r.x = NEG ? a.x + b.y : a.x - b.y;
+  r.y = NEG ? a.y - b.x : a.y + b.x;
+  return r;
 }
 // i * a
 template <typename C> __device__ __forceinline__ C cI(C a) { C r; r.x = -a.y; r.y = a.x; return r; }
@@ -188,41 +231,31 @@ __device__ __forceinline__ void dft_small(C (&v)[R]) {
   } else if constexpr (R == 4) {
     C t0 = v[0] + v[2], t1 = v[0] - v[2], t2 = v[1] + v[3], t3 = v[1] - v[3];
     // forward: multiply t3 by -i ; inverse: by +i
-    C t3r;
-    if (INV) { t3r.x = -t3.y; t3r.y = t3.x; } else { t3r.x = t3.y; t3r.y = -t3.x; }
-    v[0] = t0 + t2; v[2] = t0 - t2; v[1] = t1 + t3r; v[3] = t1 - t3r;
+    v[0] = t0 + t2; v[2] = t0 - t2;
+    v[1] = cadd_i<!INV>(t1, t3); v[3] = cadd_i<INV>(t1, t3);
   } else if constexpr (R == 3) {
     // y0 = x0 + s, y1,2 = x0 - s/2 -+ i (sqrt3/2) d  (forward), s = x1 + x2, d = x1 - x2
     using T = decltype(v[0].x);
     const T h = (T)0.86602540378443864676;  // sin(pi/3)
-    C s = v[1] + v[2], d = v[1] - v[2];
-    C a;
-    a.x = v[0].x - (T)0.5 * s.x;
-    a.y = v[0].y - (T)0.5 * s.y;
-    C t;  // -i h d (forward) or +i h d (inverse)
-    if (INV) { t.x = -h * d.y; t.y = h * d.x; } else { t.x = h * d.y; t.y = -h * d.x; }
+    const C s = v[1] + v[2], d = v[1] - v[2];
+    const C a = rfma((T)-0.5, s, v[0]);
+    const T hs = INV ? -h : h;   // y1 = a + (hs d.y, -hs d.x), y2 = a - the same
     v[0] = v[0] + s;
-    v[1] = a + t;
-    v[2] = a - t;
+    v[1].x = fma(hs, d.y, a.x);  v[1].y = fma(-hs, d.x, a.y);
+    v[2].x = fma(-hs, d.y, a.x); v[2].y = fma(hs, d.x, a.y);
   } else if constexpr (R == 5) {
     using T = decltype(v[0].x);
     const T c1 = (T)0.30901699437494742410, c2 = (T)-0.80901699437494742410;
     const T s1 = (T)0.95105651629515357212, s2 = (T)0.58778525229247312917;
     const C s14 = v[1] + v[4], d14 = v[1] - v[4], s23 = v[2] + v[3], d23 = v[2] - v[3];
-    C a1, a2, b1, b2;
-    a1.x = v[0].x + c1 * s14.x + c2 * s23.x;  a1.y = v[0].y + c1 * s14.y + c2 * s23.y;
-    a2.x = v[0].x + c2 * s14.x + c1 * s23.x;  a2.y = v[0].y + c2 * s14.y + c1 * s23.y;
-    b1.x = s1 * d14.x + s2 * d23.x;            b1.y = s1 * d14.y + s2 * d23.y;
-    b2.x = s2 * d14.x - s1 * d23.x;            b2.y = s2 * d14.y - s1 * d23.y;
+    const C a1 = rfma(c2, s23, rfma(c1, s14, v[0])), a2 = rfma(c1, s23, rfma(c2, s14, v[0]));
+    const C b1 = rfma(s2, d23, s1 * d14), b2 = rfma(-s1, d23, s2 * d14);
     // forward: y1 = a1 - i b1, y4 = a1 + i b1, y2 = a2 - i b2, y3 = a2 + i b2
-    C ib1, ib2;
-    if (INV) { ib1.x = b1.y; ib1.y = -b1.x; ib2.x = b2.y; ib2.y = -b2.x; }   // -(i b)
-    else { ib1.x = -b1.y; ib1.y = b1.x; ib2.x = -b2.y; ib2.y = b2.x; }      // +(i b)
     v[0] = v[0] + s14 + s23;
-    v[1] = a1 - ib1;
-    v[4] = a1 + ib1;
-    v[2] = a2 - ib2;
-    v[3] = a2 + ib2;
+    v[1] = cadd_i<!INV>(a1, b1);
+    v[4] = cadd_i<INV>(a1, b1);
+    v[2] = cadd_i<!INV>(a2, b2);
+    v[3] = cadd_i<INV>(a2, b2);
   } else {
     // any other prime factor (7, 11, ..., 31: bandlimits and grids off the
     // 2/3/5 sizes): a direct DFT, its outer loop kept rolled so that the code
@@ -368,8 +401,7 @@ __device__ __forceinline__ void fft_lane_pair(C (&x)[H], int h) {
   for (int k = 0; k < H; ++k) {
     const T ox = __shfl_xor_sync(pm, x[k].x, 1);
     const T oy = __shfl_xor_sync(pm, x[k].y, 1);
-    x[k].x = fma(sg, x[k].x, ox);
-    x[k].y = fma(sg, x[k].y, oy);
+    x[k] = rfma(sg, x[k], mk(ox, oy));
   }
 }
 
