@@ -72,8 +72,8 @@ struct hp_plan {
   int beta_engine = 0;
   // launch shapes chosen by hp_plan_autotune (defaults: the hand-picked ones)
   struct Tune {
-    int synth_pt = 1;      // omega points per beta-stage item of the synthesis (1, 2, 4; FP32)
-    int synth_waves = 8;   // resident waves of synthesis blocks per SM set
+    int synth_pt = 1;      // kept for the interface and saved files; no kernel takes it
+    int synth_waves = 8;   // resident waves of one-pass synthesis blocks per SM set
     int tc_waves = 16;     // waves of tensor-core CTAs of the forward beta contraction
     int tc_form = 0;       // 0: the staged tensor-core kernel, 1: the warp-specialised TMA-fed one
   } tune;

@@ -1,0 +1,286 @@
+// Synthesis in two passes (ifftSO3R.m:16-37), for complex plans and for the
+// real ones that the rule of RealSynthCfg leaves out: bandlimits whose tables
+// and buffers do not fit the one-pass kernel, and the smallest.  Included by
+// transform_b.cuh.
+//   k_synth_beta  warp = one (m, n) pair x 32 omega points: the pair's l-run of
+//                 coefficients stays in registers, every beta's sum
+//                 G_b[m][n] = sum_l (2l+1) d^l_mn(beta_b) F^l_mn goes to G;
+//   k_synth_ga    block = NB betas x PA omega points: gamma FFT over n, alpha
+//                 FFT over m, the 2B-runs of the density leave by bulk copies.
+// What bounds it: G is written and read once (NM * 2B values per omega point
+// and beta).  The omega points are taken in chunks whose G stays in L2, so that
+// HBM sees little more than F and the density.  The one-kernel form before read
+// the coefficients of a pair again for every one or two betas and its d rows
+// from L2 for every batch; 88 % of its time at B = 32 was the latency of those
+// reads.  24 x 24 omega points, before / now (both passes): B = 32 complex FP32
+// 5.85 / 1.24 ms, FP64 14.0 / 2.40; B = 24 complex FP32 1.35 / 0.56; B = 20 real
+// FP32 0.49 / 0.16.  Where both forms exist the one-pass kernel is faster (24^3,
+// B = 12 FP32: 0.48 against 0.66 ms, B = 15 FP64: 1.93 against 2.58).
+#pragma once
+
+// G of one chunk of omega points: half of the 126 MB L2
+constexpr long long kSynthG = 64LL << 20;
+
+template <int B, typename T, bool CPLX> struct Synth2Cfg {
+  using C = c2<T>;
+  static constexpr int NB2 = 2 * B, NM = CPLX ? 2 * B - 1 : B, NCOL = CPLX ? 2 * B : B;
+  // omega points per tile: whole 32-byte sectors of G (16-byte pieces cost
+  // k_synth_beta a tenth of its time at B = 32, FP32, complex)
+  static constexpr int PA = sizeof(T) == 4 ? 4 : 2;
+  static constexpr int NT = NCOL * PA > 128 ? 256 : 128;
+  static constexpr int VAL = (int)sizeof(T) * (CPLX ? 2 : 1);     // bytes of a density value
+  // staging run of one (omega point, gamma column): NB lines, an odd number of
+  // 16-byte units apart
+  static constexpr int rs_bytes(int nb) { return (((nb * NB2 * VAL + 15) / 16) | 1) * 16; }
+  static constexpr long long bytes(int nb, int pa) {
+    const long long g = (long long)nb * NM * NB2 * pa * (long long)sizeof(C);
+    const long long st = (long long)pa * NB2 * rs_bytes(nb);
+    return g > st ? g : st;
+  }
+  // three blocks per SM where a tile allows it; the alpha stage is one round
+  static constexpr bool fits(int nb, int pa) { return bytes(nb, pa) <= 72 * 1024 && nb * NCOL * pa <= NT; }
+  static constexpr int pick_nb() {
+    int nb = 1;
+    while (nb < 8 && nb < NB2 && fits(nb + 1, PA)) ++nb;
+    return nb;
+  }
+  static constexpr int NB = pick_nb();
+  // blocks per SM the registers allow
+  static constexpr int MINB = NT == 256 ? 1 : sizeof(T) == 8 ? 2 : (NB2 <= 24 ? 5 : NB2 <= 40 ? 4 : 2);
+};
+
+// dtab: [row][DS] (2l+1) d^l_mn(beta_b), DS = 2B rounded up to 4; Fp: [row][nx];
+// G: [w / PA][b][m][n bin ^ x(m)][w % PA] of the chunk's omega points.
+template <int B, typename T, bool CPLX>
+__global__ void __launch_bounds__(128) k_synth_beta(long long nx, const c2<T>* __restrict__ Fp,
+                                                    const T* __restrict__ dtab, const int2* __restrict__ pairs,
+                                                    int npairs, c2<T>* __restrict__ G, long long w0, long long nwc) {
+  using C = c2<T>;
+  using Cfg = Synth2Cfg<B, T, CPLX>;
+  constexpr int NB2 = 2 * B, NM = Cfg::NM, PA = Cfg::PA, DS = (NB2 + 3) / 4 * 4;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int lane = threadIdx.x & 31, pi = blockIdx.y * 4 + (threadIdx.x >> 5);
+  if (pi >= npairs) return;
+  const int2 pe = pairs[pi];
+  const int s = pe.x, len = pe.y & 0xff, mi = (pe.y >> 8) & 0xff, q = (pe.y >> 16) & 0xff;
+  // the warp's table rows (whole groups of four: the rows past the run multiply
+  // zero coefficients) go to shared memory in one go; read from L2 a sector at
+  // a time as the betas advance, they were the stall of three issues in four
+  T* d = reinterpret_cast<T*>(smraw) + (threadIdx.x >> 5) * ((B + 3) / 4 * 4 * DS);
+  {
+    constexpr int EPP = 16 / (int)sizeof(T);
+    const T* dsrc = dtab + (size_t)s * DS;
+    for (int e = lane; e < (len + 3) / 4 * 4 * DS / EPP; e += 32) cp_async<16>(d + e * EPP, dsrc + e * EPP, true);
+  }
+  const long long wl = (long long)blockIdx.x * 32 + lane;
+  const C* src = Fp + (size_t)s * nx + w0 + wl;
+  C v[B];
+#pragma unroll
+  for (int j = 0; j < B; ++j) v[j] = j < len && wl < nwc ? src[(size_t)j * nx] : czero<C>();
+  cp_async_wait_all();
+  __syncwarp();
+  if (wl >= nwc) return;
+  C* g = G + (((wl / PA) * NB2 * NM + mi) * NB2 + (q ^ GSwz<B, C, PA>::x(mi))) * PA + wl % PA;
+#pragma unroll 1
+  for (int b0 = 0; b0 < NB2; b0 += 4) {
+    C acc[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) acc[u] = czero<C>();
+    // four rows at a time, their table loads (one address per warp) together
+#pragma unroll
+    for (int j0 = 0; j0 < B; j0 += 4) {
+      if (j0 < len) {
+        struct alignas(16) Vec { T x[4]; };
+        Vec w[4];
+#pragma unroll
+        for (int j = 0; j < 4 && j0 + j < B; ++j) w[j] = *reinterpret_cast<const Vec*>(d + (j0 + j) * DS + b0);
+#pragma unroll
+        for (int j = 0; j < 4 && j0 + j < B; ++j)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            acc[u].x = fma(w[j].x[u], v[j0 + j].x, acc[u].x);
+            acc[u].y = fma(w[j].x[u], v[j0 + j].y, acc[u].y);
+          }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (b0 + u < NB2) g[(size_t)(b0 + u) * NM * NB2 * PA] = acc[u];
+  }
+}
+
+template <int B, typename T, bool CPLX>
+__global__ void __launch_bounds__(Synth2Cfg<B, T, CPLX>::NT, Synth2Cfg<B, T, CPLX>::MINB)
+    k_synth_ga(const c2<T>* __restrict__ G, void* __restrict__ fout, long long w0) {
+  using C = c2<T>;
+  using Cfg = Synth2Cfg<B, T, CPLX>;
+  constexpr int NB2 = 2 * B, NM = Cfg::NM, NCOL = Cfg::NCOL, PA = Cfg::PA, NB = Cfg::NB, NT = Cfg::NT;
+  using Swz = GSwz<B, C, PA>;
+  constexpr int K = Swz::K, RS = Cfg::rs_bytes(NB);
+  extern __shared__ __align__(16) unsigned char smraw[];
+  C* sG = reinterpret_cast<C*>(smraw);
+  constexpr int NGRP = (NB2 + NB - 1) / NB;
+  const int b0 = (blockIdx.x % NGRP) * NB, nbv = min(NB, NB2 - b0);
+  const long long wb = blockIdx.x / NGRP;
+  const int tid = threadIdx.x;
+  {
+    const C* src = G + (wb * NB2 + b0) * NM * NB2 * PA;
+    constexpr int EPP = 16 / (int)sizeof(C);
+    const int n = nbv * NM * NB2 * PA / EPP;
+    for (int e = tid; e < n; e += NT) cp_async<16>(sG + e * EPP, src + (size_t)e * EPP, true);
+    cp_async_wait_all();
+  }
+  __syncthreads();
+  // gamma stage: item (bb, m, p), in place; bin B is empty
+  for (int it = tid; it < nbv * NM * PA; it += NT) {
+    const int rowi = it / PA, s = Swz::x(rowi % NM);
+    C* base = sG + (size_t)rowi * NB2 * PA + it % PA;
+    C* cls[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) cls[k] = base + (k ^ s) * PA;
+    C x[NB2];
+#pragma unroll
+    for (int j = 0; j < NB2; ++j) x[j] = j == B ? czero<C>() : cls[j % K][(j / K * K) * PA];
+    fft<NB2, false>(x);
+#pragma unroll
+    for (int j = 0; j < NB2; ++j) cls[j % K][(j / K * K) * PA] = x[j];
+  }
+  __syncthreads();
+  // alpha stage, one round.  Real plans: two columns c, c + B per complex FFT
+  // (the Hermitian extensions of H[.][c]); complex plans: one column.
+  const int p = tid % PA, c = (tid / PA) % NCOL, bb = tid / (PA * NCOL);
+  const bool act = bb < nbv;
+  C x[NB2];
+  if (act) {
+    const C* h = sG + (size_t)bb * NM * NB2 * PA + p;
+    x[B] = czero<C>();
+    if constexpr (CPLX) {
+#pragma unroll
+      for (int mi = 0; mi < NM; ++mi) {
+        const int m = mi - (B - 1);
+        x[m >= 0 ? m : m + NB2] = h[(mi * NB2 + (c ^ Swz::x(mi))) * PA];
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < B; ++m) {
+        const C u = h[(m * NB2 + (c ^ Swz::x(m))) * PA], v = h[(m * NB2 + ((c + B) ^ Swz::x(m))) * PA];
+        if (m == 0) {
+          x[0] = mk(u.x, v.x);
+        } else {
+          x[m] = cadd_i<false>(u, v);
+          x[NB2 - m] = mk(u.x + v.y, v.x - u.y);
+        }
+      }
+    }
+    fft<NB2, false>(x);
+  }
+  __syncthreads();
+  if (act) {   // staging runs [c][p] of nbv lines, aliasing sG
+    unsigned char* st = smraw + (size_t)(c * PA + p) * RS;
+    if constexpr (CPLX) {
+      C* o = reinterpret_cast<C*>(st) + bb * NB2;
+#pragma unroll
+      for (int a = 0; a < NB2; ++a) o[a] = x[a];
+    } else {
+      T* o = reinterpret_cast<T*>(st) + bb * NB2;
+      T* o2 = reinterpret_cast<T*>(st + (size_t)B * PA * RS) + bb * NB2;
+      if constexpr (sizeof(T) == 4) {
+        if (((bb * NB2) & 3) == 0) stage_run<NB2, 0>(o, o2, x);
+        else stage_run<NB2, 2>(o, o2, x);
+      } else {
+#pragma unroll
+        for (int i = 0; i < NB2; i += 2) {
+          *reinterpret_cast<double2*>(o + i) = make_double2(x[i].x, x[i + 1].x);
+          *reinterpret_cast<double2*>(o2 + i) = make_double2(x[i].y, x[i + 1].y);
+        }
+      }
+    }
+  }
+  // bulk copies where every run starts and ends on a 16-byte boundary
+  constexpr int VAL = Cfg::VAL;
+  const bool bulk = (reinterpret_cast<unsigned long long>(fout) & 15ull) == 0 && (b0 * NB2 * VAL) % 16 == 0 &&
+                    (nbv * NB2 * VAL) % 16 == 0 && (NB2 * NB2 * VAL) % 16 == 0;
+  if (bulk) fence_proxy_async_smem();
+  __syncthreads();
+  // f[a + 2B (b + 2B (c + 2B w))]
+  auto dst = [&](int run) -> unsigned char* {
+    const long long w = w0 + wb * PA + run % PA;
+    return reinterpret_cast<unsigned char*>(fout) + (((size_t)w * NB2 + run / PA) * NB2 + b0) * NB2 * VAL;
+  };
+  if (bulk) {
+    const uint64_t pol = l2_policy_evict_first();
+    if ((tid & 31) == 0)
+      for (int run = tid >> 5; run < PA * NB2; run += NT / 32)
+        bulk_s2g(dst(run), smraw + (size_t)run * RS, (unsigned)(nbv * NB2 * VAL), pol);
+    bulk_commit();
+    bulk_wait_all();   // shared memory must outlive the copies reading it
+  } else {
+    for (int run = tid >> 5; run < PA * NB2; run += NT / 32) {
+      T* o = reinterpret_cast<T*>(dst(run));
+      const T* src = reinterpret_cast<const T*>(smraw + (size_t)run * RS);
+      for (int e = tid & 31; e < nbv * NB2 * (VAL / (int)sizeof(T)); e += 32) o[e] = src[e];
+    }
+  }
+}
+
+// (2l+1) d^l_mn(beta_b) as [row][DS], zero beyond b = 2B and in B more rows
+// (k_synth_beta reads whole groups of four rows)
+template <typename T>
+__global__ void k_dsyn_table(RowLayout L, const T* __restrict__ wig, int DS, T* __restrict__ out) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= (L.nrows + L.B) * DS) return;
+  const long long r = t / DS;
+  const int b = (int)(t % DS);
+  out[t] = r < L.nrows && b < 2 * L.B ? (T)(2 * L.rows[r].x + 1) * wig[(size_t)b * L.nrows + r] : (T)0;
+}
+
+template <int B, typename T, bool CPLX>
+int synth2_launch(hp_plan* p, const c2<T>* Fp, void* f, cudaStream_t s) {
+  using C = c2<T>;
+  using Cfg = Synth2Cfg<B, T, CPLX>;
+  constexpr int NB2 = 2 * B, NM = Cfg::NM, PA = Cfg::PA, NB = Cfg::NB, NPAIR = NM * (2 * B - 1), DS = (NB2 + 3) / 4 * 4;
+  int st = HP_OK;
+  const char* key = CPLX ? "tf.pairs_c" : "tf.pairs_r";
+  bool have = false;
+  for (auto& kv : p->ws) if (kv.first == key) have = true;
+  int2* dpairs = (int2*)p->ws_get(key, sizeof(int2) * NPAIR, &st);
+  if (st) return st;
+  if (!have) {
+    st = build_pairs<B, CPLX>(p, dpairs);
+    if (st) return st;
+  }
+  const char* dkey = sizeof(T) == 8 ? "tf.dsyn64" : "tf.dsyn32";
+  have = false;
+  for (auto& kv : p->ws) if (kv.first == dkey) have = true;
+  T* dtab = (T*)p->ws_get(dkey, sizeof(T) * (p->nrows + B) * DS, &st);
+  if (st) return st;
+  if (!have) {
+    const long long n = (p->nrows + B) * DS;
+    k_dsyn_table<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
+        p->layout(), sizeof(T) == 8 ? (const T*)(const void*)p->wig64 : (const T*)(const void*)p->wig32, DS, dtab);
+    HP_CUDA_TRY(cudaGetLastError());
+  }
+  const long long per_w = (long long)NM * NB2 * NB2 * (long long)sizeof(C);
+  long long nwc = std::max(32LL, kSynthG / per_w / 32 * 32);
+  nwc = std::min(nwc, (p->nx + 31) / 32 * 32);
+  C* G = (C*)p->ws_get("tf.G", (size_t)per_w * nwc, &st);
+  if (st) return st;
+  constexpr size_t smem = (size_t)Cfg::bytes(NB, PA);
+  HP_CUDA_TRY(cudaFuncSetAttribute(k_synth_ga<B, T, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  constexpr int NGRP = (NB2 + NB - 1) / NB;
+  for (long long w0 = 0; w0 < p->nx; w0 += nwc) {
+    const long long nw = std::min(nwc, p->nx - w0);   // a multiple of 4 (N is even), so of PA
+    {
+      ProfScope _ps(p, "tf.synth.beta", s);
+      constexpr size_t dsm = 4 * sizeof(T) * (size_t)((B + 3) / 4 * 4 * DS);
+      HP_CUDA_TRY(cudaFuncSetAttribute(k_synth_beta<B, T, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm));
+      k_synth_beta<B, T, CPLX><<<dim3((unsigned)((nw + 31) / 32), (unsigned)((NPAIR + 3) / 4)), 128, dsm, s>>>(
+          p->nx, Fp, dtab, dpairs, NPAIR, G, w0, nw);
+      HP_CUDA_TRY(cudaGetLastError());
+    }
+    ProfScope _ps(p, "tf.synth", s);
+    k_synth_ga<B, T, CPLX><<<(unsigned)(nw / PA * NGRP), Cfg::NT, smem, s>>>(G, f, w0);
+    HP_CUDA_TRY(cudaGetLastError());
+  }
+  return HP_OK;
+}

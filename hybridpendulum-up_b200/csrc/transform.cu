@@ -22,52 +22,61 @@ using namespace hp;
 
 // ------------------------------------------------------------ omega FFTs ----
 
-// Omega-blocked layout of the synthesis input: blocks of blk consecutive omega
-// points, each block holding every row's blk values contiguously,
-// [w / blk][row][w % blk].  One synthesis batch (blk = P omega points) then
-// reads a single contiguous run of nrows * P values, and the rows of one
-// (m, n) pair (consecutive in l) sit P values apart.  FP64 synthesis reads
-// this layout (B = 15, 32^3: 9.0 ms per synthesis against 10.0 from
-// [row][omega], while the blocked omega-FFT stores cost 0.35 ms more); FP32
-// synthesis reads [row][omega] (the same 2.85 ms either way, and the blocked
-// stores would cost 0.5 ms more).
-__host__ __device__ __forceinline__ long long omega_block_index(long long w, long long row, long long nrows, int blk) {
-  return (w / blk * nrows + row) * blk + w % blk;
+// Omega-blocked layout of the one-pass synthesis's input (synth.cuh): blocks of
+// blk (4 FP32 or 2 to 4 FP64, a divisor of N^2) consecutive omega points, each
+// block holding every row's blk values contiguously, [w / blk][row][w % blk].
+// One synthesis batch (blk = P omega points) is then a single contiguous run of
+// nrows * P values.  B = 15, 24^3, FP32: synthesis 1025 -> 882 us for 20 us more
+// in the plane pass's stores.
+
+// Distance of two planes in shared memory: N rows of N + 1 values, padded so
+// that the rows' pieces of one omega block (4 FP32 or 2 FP64 points each) sit
+// on distinct banks when the blocked store reads them one after another
+// (B = 15, 32^3, FP32: 0.29 -> 0.2 ms).
+template <int N, typename T> __host__ __device__ constexpr int wplane_ps() {
+  constexpr int U = sizeof(T) == 4 ? 16 : 8, r = (N * (N + 1)) % U;   // values per 128-byte wavefront
+  return N * (N + 1) + (U / 4 - r + U) % U;
 }
 
 // Planes per block of k_wplane: enough that the N FFTs of each pass of every
 // plane give the 128 threads one FFT each, within 64 KB of shared memory.
 template <int N, typename T> __host__ __device__ constexpr int wplane_ppb() {
   constexpr int want = 128 / N > 1 ? 128 / N : 1;
-  constexpr int fit = (int)((64 * 1024) / ((size_t)N * (N + 1) * sizeof(c2<T>)));
+  constexpr int fit = (int)((64 * 1024) / ((size_t)wplane_ps<N, T>() * sizeof(c2<T>)));
   return want < fit ? want : (fit > 1 ? fit : 1);
 }
 
 // 2-D FFT over (k1, k2) of every (row, k3) plane; PPB consecutive planes (one
 // contiguous run of PPB N^2 values) per block.
 // blk > 0: the output goes to the omega-blocked layout of the synthesis input
-// (see omega_block_index), plane pl holding omega points pl_w0 .. pl_w0 + N^2 of
-// row pl / planes_per_row.  in may equal out (a block reads all of its planes
-// before it writes).
+// (above); the block's planes are then the same k3 plane of PPB
+// consecutive rows, whose blk-point pieces are neighbours in that layout.  in
+// may equal out for blk = 0 (a block reads all of its planes before it writes).
 template <int N, typename Tin, typename T, bool INV>
 __global__ void __launch_bounds__(128) k_wplane(const c2<Tin>* __restrict__ in, c2<T>* __restrict__ out,
                                                 long long nplanes, T scale, int blk = 0, long long nrows = 0,
                                                 int planes_per_row = 1) {
   using C = c2<T>;
   constexpr int PPB = wplane_ppb<N, T>();
-  constexpr int PS = N * (N + 1);
+  constexpr int PS = wplane_ps<N, T>();
   extern __shared__ __align__(16) unsigned char smraw[];
-  C* sm = reinterpret_cast<C*>(smraw);   // [PPB][N][N+1]
-  const long long pl0 = (long long)blockIdx.x * PPB;
+  C* sm = reinterpret_cast<C*>(smraw);   // [PPB][N][N+1], planes PS apart
+  // planes of the block: consecutive ones, PS0 = N^2 values apart in memory;
+  // for blocked output the same plane of consecutive rows, so that every omega
+  // block of the output gets one contiguous run of np * blk values
+  const long long rgroups = (nrows + PPB - 1) / PPB;
+  const long long pl0 = blk > 0 ? (long long)(blockIdx.x % rgroups) * PPB * planes_per_row + blockIdx.x / rgroups
+                                : (long long)blockIdx.x * PPB;
+  const long long PS0 = blk > 0 ? (long long)N * N * planes_per_row : (long long)N * N;
   if (pl0 >= nplanes) return;
-  const int np = (int)min((long long)PPB, nplanes - pl0);
+  const int np = (int)min((long long)PPB, blk > 0 ? nrows - pl0 / planes_per_row : nplanes - pl0);
   const int tot = np * N * N;
   const c2<Tin>* src = in + pl0 * N * N;
   if constexpr (sizeof(Tin) == sizeof(T)) {
     // no conversion: the block's whole run is in flight at once (cp.async,
     // no register round trip)
     for (int e = threadIdx.x; e < tot; e += blockDim.x)
-      cp_async<sizeof(C)>(sm + (e / (N * N)) * PS + ((e / N) % N) * (N + 1) + e % N, src + e, true);
+      cp_async<sizeof(C)>(sm + (e / (N * N)) * PS + ((e / N) % N) * (N + 1) + e % N, src + (e / (N * N)) * PS0 + e % (N * N), true);
     cp_async_wait_all();
   } else {
     for (int e0 = threadIdx.x; e0 < tot; e0 += 4 * blockDim.x) {
@@ -75,7 +84,7 @@ __global__ void __launch_bounds__(128) k_wplane(const c2<Tin>* __restrict__ in, 
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int e = e0 + u * blockDim.x;
-        v[u] = e < tot ? cvt<C, c2<Tin>>(src[e]) : czero<C>();
+        v[u] = e < tot ? cvt<C, c2<Tin>>(src[(e / (N * N)) * PS0 + e % (N * N)]) : czero<C>();
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -106,11 +115,22 @@ __global__ void __launch_bounds__(128) k_wplane(const c2<Tin>* __restrict__ in, 
   }
   __syncthreads();
   if (blk > 0) {
-    for (int e = threadIdx.x; e < tot; e += blockDim.x) {
-      const long long pl = pl0 + e / (N * N);
-      const int q = e % (N * N);
-      const long long row = pl / planes_per_row, w0 = (pl % planes_per_row) * (long long)(N * N);
-      out[omega_block_index(w0 + q, row, nrows, blk)] = sm[(e / (N * N)) * PS + (q / N) * (N + 1) + q % N];
+    const long long row0 = pl0 / planes_per_row, w0 = (pl0 % planes_per_row) * (long long)(N * N);
+    // blocks do not straddle planes: consecutive threads write consecutive
+    // values (row, w % blk) of one block
+    const int lb = __ffs(blk) - 1;
+    const unsigned nr = (unsigned)nrows;            // N^2 nrows < 2^32 values per plane
+    C* dst = out + (((w0 >> lb) * nrows + row0) << lb);
+    auto put = [&](unsigned ob, unsigned r, unsigned t) {   // omega block of the plane, row of the group, point
+      const unsigned q = (ob << lb) + t;
+      dst[((ob * nr + r) << lb) + t] = sm[r * PS + q + q / N];
+    };
+    if (np == PPB) {
+#pragma unroll 4
+      for (unsigned e = threadIdx.x; e < (unsigned)(PPB * N * N); e += 128)
+        put((e >> lb) / PPB, (e >> lb) % PPB, e & (blk - 1));
+    } else {
+      for (int e = threadIdx.x; e < tot; e += 128) put((e >> lb) / np, (e >> lb) % np, e & (blk - 1));
     }
     return;
   }
@@ -130,11 +150,14 @@ __global__ void __launch_bounds__(128) k_wline(const c2<T>* __restrict__ in, c2<
   const long long row = t / plane, p = t % plane;
   C x[N];
   if (blk > 0) {
+    // blocks do not straddle planes: value (p, row) of plane j is number t of
+    // the plane's values, in the order of the layout
+    const long long ps = plane * nrows;
 #pragma unroll
-    for (int j = 0; j < N; ++j) x[j] = in[omega_block_index(j * plane + p, row, nrows, blk)];
+    for (int j = 0; j < N; ++j) x[j] = in[t + j * ps];
     fft<N, INV>(x);
 #pragma unroll
-    for (int j = 0; j < N; ++j) out[omega_block_index(j * plane + p, row, nrows, blk)] = scale * x[j];
+    for (int j = 0; j < N; ++j) out[t + j * ps] = scale * x[j];
     return;
   }
   const C* src = in + row * plane * N + p;
@@ -163,8 +186,8 @@ static int omega_fft(hp_plan* p, const c2<Tin>* in, c2<T>* out, bool inv, cudaSt
   const int ppr = p->ndim == 3 ? N : 1;
   const long long nplanes = p->nrows * ppr;
   constexpr int PPB = wplane_ppb<N, T>();
-  const size_t smem = sizeof(c2<T>) * PPB * N * (N + 1);
-  const unsigned nblk = (unsigned)((nplanes + PPB - 1) / PPB);
+  const size_t smem = sizeof(c2<T>) * PPB * wplane_ps<N, T>();
+  const unsigned nblk = (unsigned)(blk > 0 ? (p->nrows + PPB - 1) / PPB * ppr : (nplanes + PPB - 1) / PPB);
   auto plane = [&](T sc) -> int {
     ProfScope _ps(p, "tf.wplane", s);
     if (inv) {
@@ -218,16 +241,15 @@ static int omega_fft_any(hp_plan* p, const c2<Tin>* in, c2<T>* out, bool inv, cu
 HP_FOR_EACH_B(X)
 #undef X
 
-// Omega block of the synthesis input (P of the synthesis configuration) for
-// FP64 synthesis; 0 (the [row][omega] layout) for FP32.
+// Omega block of the synthesis input: P of the one-pass kernel, 0 (the
+// [row][omega] layout) for the two-pass one.
 template <typename T, bool CPLX>
 static int synth_block(const hp_plan* p) {
-  if (sizeof(T) == 4) return 0;
   switch (p->B) {
-#define X(b) case b: return SynthCfg<b, T, CPLX>::P;
+#define X(b) case b: return !CPLX && RealSynthCfg<b, T>::ok ? RealSynthCfg<b, T>::P : 0;
     HP_FOR_EACH_B(X)
 #undef X
-    default: return 1;
+    default: return 0;
   }
 }
 
@@ -245,15 +267,14 @@ static int synth_any(hp_plan* p, const c2<T>* Fp, void* f, cudaStream_t s) {
 
 
 // Inverse omega FFT of every row into the synthesis input (a plan workspace;
-// omega-blocked and sized for whole blocks for FP64, [row][omega] for FP32),
+// omega-blocked or [row][omega], see synth_block),
 // then the synthesis.
 template <typename Tin, typename T>
 static int backward_rows(hp_plan* p, const c2<Tin>* Fint, void* f, int complex_out, cudaStream_t s) {
   using C = c2<T>;
   int st = HP_OK;
   const int blk = complex_out ? synth_block<T, true>(p) : synth_block<T, false>(p);
-  const long long nxb = blk ? (p->nx + blk - 1) / blk * blk : p->nx;
-  const size_t fb = sizeof(C) * (size_t)p->nrows * nxb;
+  const size_t fb = sizeof(C) * (size_t)p->nrows * p->nx;   // nx is a multiple of 4
   C* t1 = (C*)p->ws_get("tf.t1", fb, &st);
   if (st) return st;
   st = omega_fft_any<Tin, T>(p, Fint, t1, true, s, blk);

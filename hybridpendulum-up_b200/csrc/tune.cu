@@ -109,20 +109,18 @@ extern "C" int hp_plan_autotune(hp_plan* p, double* best_backward_ms, double* be
   const hp_plan::Tune start = p->tune;
   hp_plan::Tune best = start;
   float best_b = 1e30f;
-  const std::vector<int> pts = p->precision == HP_FP64 ? std::vector<int>{1} : std::vector<int>{1, 2, 4};
-  for (int pt : pts)
-    for (int waves : {4, 8, 16}) {
-      p->tune.synth_pt = pt;
-      p->tune.synth_waves = waves;
-      float ms = 0;
-      const int st = time_it(s, 3, [&] { return hp_backward_internal(p, (const double2*)F.p, f.p, cplx, s); }, &ms);
-      if (st) { p->tune = start; return st; }
-      if (ms < best_b) {
-        best_b = ms;
-        best.synth_pt = pt;
-        best.synth_waves = waves;
-      }
+  for (int waves : {4, 8, 16}) {
+    p->tune.synth_pt = 1;   // no kernel takes this knob now
+    p->tune.synth_waves = waves;
+    float ms = 0;
+    const int st = time_it(s, 3, [&] { return hp_backward_internal(p, (const double2*)F.p, f.p, cplx, s); }, &ms);
+    if (st) { p->tune = start; return st; }
+    if (ms < best_b) {
+      best_b = ms;
+      best.synth_pt = 1;
+      best.synth_waves = waves;
     }
+  }
   p->tune = best;
   float best_f = 0;
   const bool tc = p->precision == HP_MIXED && hp::tc_beta_supported(p) &&

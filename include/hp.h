@@ -137,9 +137,10 @@ int hp_plan_set_beta_engine(hp_plan* plan, int engine);
 int hp_plan_tc_errors(hp_plan* plan, int* count);
 
 /* Launch-shape tuning (no counterpart in the reference).  The knobs are the
- * runtime launch shapes of the transforms: synth_pt, the omega points per item
- * of the synthesis beta stage (1, 2 or 4; FP32 plans), synth_waves, the
- * resident waves of synthesis blocks (how many omega chunks a block walks),
+ * runtime launch shapes of the transforms: synth_pt (1, 2 or 4; accepted and
+ * kept, but the present synthesis kernels do not take it), synth_waves, the
+ * resident waves of one-pass synthesis blocks (how many omega batches a block
+ * walks),
  * tc_waves, the waves of tensor-core CTAs of the forward beta contraction, and
  * tc_form, its kernel (1: the warp-specialised pipeline fed by TMA tensor
  * copies, 0: the staged single-warpgroup kernel).
