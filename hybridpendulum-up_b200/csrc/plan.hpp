@@ -152,7 +152,12 @@ void hp_tune_apply_cached(hp_plan* p);
 int hp_tables_build(hp_plan* p);
 int hp_twiddles_init();
 int hp_build_gravity_taps(hp_plan* p);
+// the weights of W Grav W^-1, W = diag(2l+1), in the plan's compute precision (out: [row][9])
+int hp_adjoint_gravity_taps(hp_plan* p, void* out, cudaStream_t s);
 int hp_full_to_internal(hp_plan* p, const double2* Ffull, double2* Fint, cudaStream_t s);
+// the same of the projection onto the real-density subspace, (F + C F) / 2
+int hp_full_to_internal_sym(hp_plan* p, const double2* Ffull, double2* Fint, cudaStream_t s);
+int hp_tables_on_grid(hp_plan* p, int Bg, double* fact, double* d, double* w, cudaStream_t s);
 int hp_internal_to_full(hp_plan* p, const double2* Fint, double2* Ffull, cudaStream_t s);
 // full layout -> [row][omega], reading only the kept entries of Ff, which may be
 // host memory mapped into the device address space (read in place)

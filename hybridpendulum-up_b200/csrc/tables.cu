@@ -35,6 +35,7 @@ int hp_twiddles_init() {
 // run for that entry: closed form at l = -n, two-term step at l = -n+1, the
 // three-term recursion above; the l = 1 entry of (0,0) is cos(beta) as in
 // Wigner_d.m:17-21.
+// B sets the nodes, lmax the degrees; the row tables are skipped where wig64 is null.
 __global__ void k_wigner(int B, int lmax, const double* __restrict__ fact, double* __restrict__ wfull,
                          RowLayout L, double* __restrict__ wig64, float* __restrict__ wig32) {
   const int D = 2 * lmax + 1;
@@ -77,7 +78,7 @@ __global__ void k_wigner(int B, int lmax, const double* __restrict__ fact, doubl
     dm1 = v;
     const double out = sign * v;
     wfull[(m + lmax) + (long long)D * (n + lmax) + (long long)D * D * l + wstride * b] = out;
-    if (m >= L.m_lo) {
+    if (wig64 && m >= L.m_lo) {
       const int am = abs(m), an = abs(n);
       const long long row = L.seg[(m - L.m_lo) * D + n + lmax] + l - (am > an ? am : an);
       wig64[(long long)b * L.nrows + row] = out;
@@ -122,7 +123,8 @@ __global__ void k_cg1(int lmax, double* cg1) {
 // weight factors into a real part per tap, stored here as
 // tap_wr[row*9 + (l1-l+1)*3 + (n2+1)] (zero where the source row does not
 // exist), and the model's MR_i^1_{0 n2}, applied per omega point.
-template <typename T>
+// ADJ: the weights of W Grav W^-1 with W = diag(2l+1), the adjoint's gravity.
+template <typename T, bool ADJ = false>
 __global__ void k_gravity_taps(RowLayout L, const double* __restrict__ cg1, T* __restrict__ tap_wr) {
   const long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (r >= L.nrows) return;
@@ -135,33 +137,68 @@ __global__ void k_gravity_taps(RowLayout L, const double* __restrict__ cg1, T* _
     if (l1 >= 0 && l1 <= lmax && abs(m) <= l1 && abs(n1) <= l1) {
       const double cm = cg1[cg1_index(lmax, l1, l - l1, m, 0)];
       const double cn = cg1[cg1_index(lmax, l1, l - l1, n, n2)];
-      w = (2.0 * l1 + 1.0) * 3.0 / (2.0 * l + 1.0) * cm * cn;
+      w = ADJ ? 3.0 * cm * cn : (2.0 * l1 + 1.0) * 3.0 / (2.0 * l + 1.0) * cm * cn;
     }
     tap_wr[r * 9 + t] = (T)w;
   }
 }
 
 // ------------------------------------------------ layout conversions ----
-// full (MATLAB F(m,n,l,w)) -> internal rows; tiles of 32 full indices x 32 omega.
-__global__ void k_full_to_int(RowLayout L, const double2* __restrict__ Ff, double2* __restrict__ Fi) {
+__device__ __forceinline__ long long mirror_w(long long w, int N, int ndim) {
+  long long r = 0, mul = 1;
+  for (int a = 0; a < ndim; ++a) {
+    const int k = (int)(w % N);
+    w /= N;
+    r += mul * ((N - k) % N);
+    mul *= N;
+  }
+  return r;
+}
+
+// full (MATLAB F(m,n,l,w)) -> internal rows; tiles of 32 kept entries x 32
+// omega.  Lanes read along the kept entries in full-layout order (adjacent m
+// are adjacent in memory) and write along omega; only the kept entries are
+// read, a fifth of the array for real plans (with the whole array read and an
+// index division per value, B = 10, 30^3: 0.6 ms; now 0.1 ms).
+// SYM: the entry is (F + C F) / 2, C the real-density mirror
+// F^l_mn[k] -> (-1)^(m-n) conj F^l_{-m,-n}[-k], so that the rows with m >= 0
+// hold the projection of F onto the real-density subspace.
+template <bool SYM>
+__global__ void k_full_to_int(const int2* __restrict__ fg, const char4* __restrict__ rows, int nrows, int lmax, int N,
+                              int ndim, long long nx, const double2* __restrict__ Ff, double2* __restrict__ Fi) {
   __shared__ double2 tile[32][33];
-  const int D = 2 * L.lmax + 1;
-  const long long Dfull = (long long)D * D * (L.lmax + 1);
-  const long long fi0 = (long long)blockIdx.x * 32, w0 = (long long)blockIdx.y * 32;
+  const int D = 2 * lmax + 1;
+  const long long Dfull = (long long)D * D * (lmax + 1);
+  const int e0 = blockIdx.x * 32;
+  const long long w0 = (long long)blockIdx.y * 32;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  for (int k = ty; k < 32; k += blockDim.y) {
-    const long long fi = fi0 + tx, w = w0 + k;
-    tile[k][tx] = (fi < Dfull && w < L.nx) ? Ff[fi + Dfull * w] : make_double2(0, 0);
+  const int e = e0 + tx;
+  const int2 g = e < nrows ? fg[e] : make_int2(0, 0);
+  int gm = 0;            // the mirrored entry and its sign
+  double sg = 1.0;
+  if (SYM && e < nrows) {
+    const char4 q = rows[g.y];
+    gm = (lmax - q.y) + D * (lmax - q.z) + D * D * q.x;
+    sg = ((q.y - q.z) & 1) ? -1.0 : 1.0;
+  }
+#pragma unroll
+  for (int k = ty; k < 32; k += 8) {
+    const long long w = w0 + k;
+    double2 v = make_double2(0, 0);
+    if (e < nrows && w < nx) {
+      v = Ff[g.x + Dfull * w];
+      if (SYM) {
+        const double2 u = Ff[gm + Dfull * mirror_w(w, N, ndim)];
+        v = make_double2(0.5 * (v.x + sg * u.x), 0.5 * (v.y - sg * u.y));
+      }
+    }
+    tile[k][tx] = v;
   }
   __syncthreads();
-  for (int k = ty; k < 32; k += blockDim.y) {
-    const long long fi = fi0 + k, w = w0 + tx;
-    if (fi >= Dfull || w >= L.nx) continue;
-    const int m = (int)(fi % D) - L.lmax, n = (int)((fi / D) % D) - L.lmax, l = (int)(fi / (D * D));
-    const int am = abs(m), an = abs(n);
-    if (am > l || an > l || m < L.m_lo) continue;
-    const long long row = L.seg[(m - L.m_lo) * D + n + L.lmax] + l - (am > an ? am : an);
-    Fi[row * L.nx + w] = tile[tx][k];
+#pragma unroll
+  for (int k = ty; k < 32; k += 8) {
+    const long long w = w0 + tx;
+    if (e0 + k < nrows && w < nx) Fi[(long long)fg[e0 + k].y * nx + w] = tile[tx][k];
   }
 }
 
@@ -183,61 +220,67 @@ __global__ void k_full_gather(const int2* __restrict__ fg, int nrows, long long 
   }
 }
 
-__device__ __forceinline__ long long mirror_w(long long w, int N, int ndim) {
-  long long r = 0, mul = 1;
-  for (int a = 0; a < ndim; ++a) {
-    const int k = (int)(w % N);
-    w /= N;
-    r += mul * ((N - k) % N);
-    mul *= N;
-  }
-  return r;
-}
-
 // internal -> full; zero outside |m|,|n| <= l; rows with m < m_lo (HP_REAL)
-// from F^l_{mn}[k] = (-1)^(m-n) conj F^l_{-m,-n}[-k].
+// from F^l_{mn}[k] = (-1)^(m-n) conj F^l_{-m,-n}[-k].  Tiles of 32 full indices
+// x 32 omega, 8 rows of threads: lanes read along omega (one full index per
+// warp and load, so its decomposition is uniform and 32-bit) and write along
+// the full index.  Writing the whole array is the bound: B = 10, 30^3 (1.56 GB)
+// took 0.6 ms with 64-bit index divisions per value.
 __global__ void k_int_to_full(RowLayout L, const double2* __restrict__ Fi, double2* __restrict__ Ff) {
   __shared__ double2 tile[32][33];
-  const int D = 2 * L.lmax + 1;
-  const long long Dfull = (long long)D * D * (L.lmax + 1);
-  const long long fi0 = (long long)blockIdx.x * 32, w0 = (long long)blockIdx.y * 32;
+  const int D = 2 * L.lmax + 1, lmax = L.lmax;
+  const int Dfull = D * D * (lmax + 1);
+  const int fi0 = blockIdx.x * 32;
+  const long long w0 = (long long)blockIdx.y * 32;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  for (int k = ty; k < 32; k += blockDim.y) {
-    const long long fi = fi0 + k, w = w0 + tx;
-    double2 v = make_double2(0, 0);
-    if (fi < Dfull && w < L.nx) {
-      int m = (int)(fi % D) - L.lmax, n = (int)((fi / D) % D) - L.lmax;
-      const int l = (int)(fi / (D * D));
-      const int am = abs(m), an = abs(n);
-      if (am <= l && an <= l) {
-        if (m >= L.m_lo) {
-          const long long row = L.seg[(m - L.m_lo) * D + n + L.lmax] + l - (am > an ? am : an);
-          v = Fi[row * L.nx + w];
-        } else {
-          const long long row = L.seg[(-m - L.m_lo) * D + (-n) + L.lmax] + l - (am > an ? am : an);
-          v = Fi[row * L.nx + mirror_w(w, L.N, L.ndim)];
-          v.y = -v.y;
-          if ((m - n) & 1) { v.x = -v.x; v.y = -v.y; }
-        }
+  const long long w = w0 + tx;
+  const long long wm = w < L.nx && L.m_lo == 0 ? mirror_w(w, L.N, L.ndim) : 0;
+  double2 v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int fi = fi0 + ty + 8 * i;
+    v[i] = make_double2(0, 0);
+    const int l = fi / (D * D), r = fi - l * D * D, nn = r / D;
+    const int m = r - nn * D - lmax, n = nn - lmax, am = abs(m), an = abs(n);
+    if (fi < Dfull && am <= l && an <= l && w < L.nx) {
+      const int lr = l - (am > an ? am : an);
+      if (m >= L.m_lo) {
+        v[i] = Fi[(long long)(L.seg[(m - L.m_lo) * D + n + lmax] + lr) * L.nx + w];
+      } else {
+        const double2 u = Fi[(long long)(L.seg[(-m - L.m_lo) * D - n + lmax] + lr) * L.nx + wm];
+        const double sg = ((m - n) & 1) ? -1.0 : 1.0;
+        v[i] = make_double2(sg * u.x, -sg * u.y);
       }
     }
-    tile[k][tx] = v;
   }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) tile[ty + 8 * i][tx] = v[i];
   __syncthreads();
-  for (int k = ty; k < 32; k += blockDim.y) {
-    const long long fi = fi0 + tx, w = w0 + k;
-    if (fi < Dfull && w < L.nx) Ff[fi + Dfull * w] = tile[tx][k];
+  const int fo = fi0 + tx;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const long long wo = w0 + ty + 8 * i;
+    if (fo < Dfull && wo < L.nx) Ff[fo + (long long)Dfull * wo] = tile[tx][ty + 8 * i];
   }
+}
+
+static int full_to_int(hp_plan* p, const double2* Ff, double2* Fi, bool sym, cudaStream_t s) {
+  dim3 grid((unsigned)((p->nrows + 31) / 32), (unsigned)((p->nx + 31) / 32));
+  ProfScope _ps(p, "layout", s);
+  if (sym)
+    k_full_to_int<true><<<grid, dim3(32, 8), 0, s>>>(p->fgather, p->rows, (int)p->nrows, p->lmax, p->N, p->ndim, p->nx, Ff, Fi);
+  else
+    k_full_to_int<false><<<grid, dim3(32, 8), 0, s>>>(p->fgather, p->rows, (int)p->nrows, p->lmax, p->N, p->ndim, p->nx, Ff, Fi);
+  HP_CUDA_TRY(cudaGetLastError());
+  return HP_OK;
 }
 
 int hp_full_to_internal(hp_plan* p, const double2* Ff, double2* Fi, cudaStream_t s) {
-  const int D = p->D;
-  const long long Dfull = (long long)D * D * (p->lmax + 1);
-  dim3 grid((unsigned)((Dfull + 31) / 32), (unsigned)((p->nx + 31) / 32));
-  ProfScope _ps(p, "layout", s);
-  k_full_to_int<<<grid, dim3(32, 8), 0, s>>>(p->layout(), Ff, Fi);
-  HP_CUDA_TRY(cudaGetLastError());
-  return HP_OK;
+  return full_to_int(p, Ff, Fi, false, s);
+}
+
+int hp_full_to_internal_sym(hp_plan* p, const double2* Ff, double2* Fi, cudaStream_t s) {
+  return full_to_int(p, Ff, Fi, true, s);
 }
 
 int hp_full_gather(hp_plan* p, const double2* Ff, double2* Fi, cudaStream_t s) {
@@ -324,6 +367,22 @@ int hp_tables_build(hp_plan* p) {
   return HP_OK;
 }
 
+// Wigner-d of the plan's degrees and quadrature weights on the 2 Bg nodes of
+// bandlimit Bg: d (2lmax+1, 2lmax+1, lmax+1, 2Bg) with zeros outside |m|,|n| <= l,
+// w (2Bg); fact: device scratch of 2 lmax + 2 values.
+int hp_tables_on_grid(hp_plan* p, int Bg, double* fact, double* d, double* w, cudaStream_t s) {
+  std::vector<double> h(2 * p->lmax + 2, 1.0);
+  for (int k = 1; k < (int)h.size(); ++k) h[k] = h[k - 1] * k;
+  HP_CUDA_TRY(cudaMemcpyAsync(fact, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, s));
+  HP_CUDA_TRY(cudaMemsetAsync(d, 0, sizeof(double) * (size_t)p->D * p->D * p->B * 2 * Bg, s));
+  const int nth = 2 * Bg * p->D * p->D;
+  k_wigner<<<(nth + 127) / 128, 128, 0, s>>>(Bg, p->lmax, fact, d, p->layout(), nullptr, nullptr);
+  k_weights<<<1, 2 * Bg, 0, s>>>(Bg, w);
+  HP_CUDA_TRY(cudaGetLastError());
+  HP_CUDA_TRY(cudaStreamSynchronize(s));   // h is read until here; once per plan
+  return HP_OK;
+}
+
 int hp_build_gravity_taps(hp_plan* p) {
   if (p->tap_wr) return HP_OK;
   HP_CUDA_TRY(hp_dev_alloc(&p->tap_wr, sizeof(double) * 9 * p->nrows));
@@ -331,6 +390,14 @@ int hp_build_gravity_taps(hp_plan* p) {
   const unsigned g = (unsigned)((p->nrows + 127) / 128);
   k_gravity_taps<double><<<g, 128, 0, p->stream>>>(p->layout(), p->cg1, p->tap_wr);
   k_gravity_taps<float><<<g, 128, 0, p->stream>>>(p->layout(), p->cg1, p->tap_wr32);
+  HP_CUDA_TRY(cudaGetLastError());
+  return HP_OK;
+}
+
+int hp_adjoint_gravity_taps(hp_plan* p, void* out, cudaStream_t s) {
+  const unsigned g = (unsigned)((p->nrows + 127) / 128);
+  if (p->precision == HP_FP64) k_gravity_taps<double, true><<<g, 128, 0, s>>>(p->layout(), p->cg1, (double*)out);
+  else k_gravity_taps<float, true><<<g, 128, 0, s>>>(p->layout(), p->cg1, (float*)out);
   HP_CUDA_TRY(cudaGetLastError());
   return HP_OK;
 }
