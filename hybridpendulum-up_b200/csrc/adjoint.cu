@@ -16,7 +16,10 @@
 //   * (b_i D_i M_i)^H = -b_i M_i D_i (D_i = 2 pi i kappa / L is imaginary);
 //     M_i and D_i do not commute on the grid, so this term is applied as its
 //     own pass (multiply by D_i, inverse FFT, times x_i, FFT).
-// The first bracket is the forward derivative kernel with b = 0 and G -> -G.
+// The first bracket is the forward derivative kernel with b = 0, G -> -G and
+// the gravity taps of W Grav W^-1 (the other terms keep l and commute with W).
+// B = 12, 24^3, FP64: a reverse step's terms beyond its derivative evaluation
+// took 4.3 ms as 37 passes over whole arrays; now 7 passes.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -34,226 +37,248 @@ using namespace hp;
 
 namespace {
 
-constexpr int kDotThreads = 256;
 constexpr int kDotBlocks = 592;  // 4 per SM
 
-// out = (add ? lam : 0) - a * (2l+1) * d1
-__global__ void k_adj_combine(RowLayout L, const double2* __restrict__ lam, const double2* __restrict__ d1,
-                              double2* __restrict__ out, double a, int add) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= L.nrows * L.nx) return;
-  const int l = L.rows[t / L.nx].x;
-  const double s = a * (2 * l + 1);
-  const double2 v = d1[t];
-  double2 o = add ? lam[t] : make_double2(0.0, 0.0);
-  o.x -= s * v.x;
-  o.y -= s * v.y;
-  out[t] = o;
+// Lines of N points along `axis` (stride N^axis inside a row), one thread per
+// line: what the axis contributes to the adjoint and to the gradients.  With
+// ifft the unnormalised inverse, u = ifft(i d lam), v = ifft(F), x the grid
+// coordinate and d = 2 pi kappa / L of this axis:
+//   dot   += scale * weight * Re<lam, D M F> = -scale * weight / N sum_j x_j Re conj(u_j) v_j
+//   out   += coef * M D lam = coef * fft(x u) / N            (out may be null)
+//   Y1, Y2 = ifft(lam), ifft(F)                              (may be null)
+// Lanes run along the contiguous omega index, so the strided axes read and
+// write whole lines; the contiguous axis (AXIS0) goes through tiles in shared
+// memory (one thread per contiguous line, straight from global memory, read
+// 16 bytes of every 16 N).  v waits in shared memory while u is formed.  One
+// pass of this kernel replaces a pass M D lam, a pass D M F and a dot.
+template <int N> __host__ __device__ constexpr int line_threads(bool axis0) {
+  return axis0 ? 64 : (N <= 32 ? 128 : 64);
+}
+template <int N> __host__ __device__ constexpr size_t line_smem(bool axis0) {
+  return sizeof(double2) * (axis0 ? 2 * (size_t)line_threads<N>(true) * (N + 1) : (size_t)line_threads<N>(false) * N);
 }
 
-// out = in / (2l+1)
-__global__ void k_row_unweight(RowLayout L, const double2* __restrict__ in, double2* __restrict__ out) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= L.nrows * L.nx) return;
-  const double s = 1.0 / (2 * L.rows[t / L.nx].x + 1);
-  const double2 v = in[t];
-  out[t] = make_double2(s * v.x, s * v.y);
-}
-
-// out += coef * M_axis (D_axis in): one thread per line of N points along
-// `axis` (stride N^axis inside a row).
-template <int N>
-__global__ void __launch_bounds__(128) k_axis_md(RowLayout L, const double2* __restrict__ in,
-                                                 double2* __restrict__ out, int axis, double coef, double Llen) {
-  const long long nlines = L.nx / N;
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= L.nrows * nlines) return;
-  const long long row = t / nlines, q = t % nlines;
-  long long stride = 1;
-  for (int a = 0; a < axis; ++a) stride *= N;
-  const long long lo = q % stride, hi = q / stride;
-  const long long base = row * L.nx + hi * stride * N + lo;
-  const double tp = 2.0 * M_PI / Llen;
-  double2 x[N];
-#pragma unroll
-  for (int j = 0; j < N; ++j) {
-    const double2 v = in[base + j * stride];
-    const double dk = tp * kappa_first(j, N);
-    x[j] = make_double2(-dk * v.y, dk * v.x);  // D v = i dk v
-  }
-  fft<N, true>(x);
-#pragma unroll
-  for (int j = 0; j < N; ++j) {
-    const double xc = (-Llen / 2 + Llen * j / N) / N;
-    x[j] = xc * x[j];
-  }
-  fft<N, false>(x);
-#pragma unroll
-  for (int j = 0; j < N; ++j) {
-    double2 o = out[base + j * stride];
-    o.x += coef * x[j].x;
-    o.y += coef * x[j].y;
-    out[base + j * stride] = o;
-  }
-}
-
-// out (=, or += with acc) coef * D_daxis (M_axis in): one thread per line of N
-// points along `axis`; M_axis multiplies by x_axis on the omega grid
-// (inverse FFT, times x, FFT), D_daxis by 2 pi i kappa / L along axis daxis
-// (any axis, applied per point after M; daxis < 0: none).
-template <int N>
-__global__ void __launch_bounds__(128) k_line_dm(RowLayout L, const double2* __restrict__ in,
-                                                 double2* __restrict__ out, int axis, int daxis, double coef,
-                                                 double Llen, int acc) {
-  const long long nlines = L.nx / N;
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= L.nrows * nlines) return;
-  const long long row = t / nlines, q = t % nlines;
-  long long stride = 1, dstride = 1;
-  for (int a = 0; a < axis; ++a) stride *= N;
-  for (int a = 0; a < daxis; ++a) dstride *= N;
-  const long long lo = q % stride, hi = q / stride;
-  const long long w0 = hi * stride * N + lo;   // omega index of the line's first point
-  const long long base = row * L.nx + w0;
-  const double tp = 2.0 * M_PI / Llen;
-  double2 x[N];
-#pragma unroll
-  for (int j = 0; j < N; ++j) x[j] = in[base + j * stride];
-  fft<N, true>(x);
-#pragma unroll
-  for (int j = 0; j < N; ++j) {
-    const double xc = (-Llen / 2 + Llen * j / N) / N;
-    x[j] = xc * x[j];
-  }
-  fft<N, false>(x);
-#pragma unroll
-  for (int j = 0; j < N; ++j) {
-    double2 v = x[j];
-    if (daxis >= 0) {   // i dk v
-      const long long w = w0 + j * stride;
-      const double dk = tp * kappa_first((int)((w / dstride) % N), N);
-      v = make_double2(-dk * v.y, dk * v.x);
-    }
-    double2 o = acc ? out[base + j * stride] : make_double2(0.0, 0.0);
-    o.x += coef * v.x;
-    o.y += coef * v.y;
-    out[base + j * stride] = o;
-  }
-}
+struct LineArgs {
+  const double2* lam;
+  const double2* F;
+  double2* out;
+  double2* Y1;
+  double2* Y2;
+  int axis;
+  double coef, scale, Llen;
+  int half, slot;
+  double* acc;
+};
 
 __device__ __forceinline__ double row_weight(const RowLayout& L, long long row, int half) {
   return (half && L.rows[row].y > 0) ? 2.0 : 1.0;
 }
 
-// acc[slot * gridDim.x + block] += scale * sum w Re(conj(a) b); one slot per call.
-__global__ void __launch_bounds__(kDotThreads) k_dot(RowLayout L, const double2* __restrict__ a,
-                                                     const double2* __restrict__ b, double* __restrict__ acc,
-                                                     int slot, double scale, int half) {
-  __shared__ double red[kDotThreads];
-  double s = 0.0;
-  const long long n = L.nrows * L.nx;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x) {
-    const double2 u = a[t], v = b[t];
-    s += row_weight(L, t / L.nx, half) * (u.x * v.x + u.y * v.y);
-  }
-  red[threadIdx.x] = s;
+// acc[slot][block] += the block's sum of v
+__device__ __forceinline__ void block_add(double v, double* acc, int slot) {
+  __shared__ double red[4];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  for (int k = kDotThreads / 2; k > 0; k >>= 1) {
-    if (threadIdx.x < k) red[threadIdx.x] += red[threadIdx.x + k];
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int k = 0; k < (int)blockDim.x / 32; ++k) t += red[k];
+    acc[(long long)slot * gridDim.x + blockIdx.x] += t;
   }
-  if (threadIdx.x == 0) acc[(long long)slot * gridDim.x + blockIdx.x] += scale * red[0];
 }
 
-// The noise-term gradients: slots slot0 + (i, j) pair index (i <= j) get
-// scale * sum w c_ij(k) Re(conj(a) b), c_ii = -(2 pi kd_i / L)^2 with the
-// Nyquist bin kept, c_ij = -(2 pi k_i / L)(2 pi k_j / L) with it zeroed
-// (pendulum.m:510-523).
-__global__ void __launch_bounds__(kDotThreads) k_dot_noise(RowLayout L, const double2* __restrict__ a,
-                                                           const double2* __restrict__ b, double* __restrict__ acc,
-                                                           int slot0, double scale, int half, double Llen) {
-  __shared__ double red[6][kDotThreads];
-  double s[6] = {0, 0, 0, 0, 0, 0};
-  const long long n = L.nrows * L.nx;
-  const int N = L.N, nd = L.ndim;
-  const double tp = 2.0 * M_PI / Llen;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x) {
-    const double2 u = a[t], v = b[t];
-    const double r = row_weight(L, t / L.nx, half) * (u.x * v.x + u.y * v.y);
-    long long w = t % L.nx;
-    double d1[3] = {0, 0, 0}, dd[3] = {0, 0, 0};
-    for (int i = 0; i < nd; ++i) {
-      const int k = (int)(w % N);
-      w /= N;
-      d1[i] = tp * kappa_first(k, N);
-      dd[i] = tp * kappa_diag(k, N);
-    }
-    int q = 0;
-    for (int i = 0; i < 3; ++i)
-      for (int j = i; j < 3; ++j, ++q) {
-        if (i >= nd || j >= nd) continue;
-        s[q] -= r * (i == j ? dd[i] * dd[i] : d1[i] * d1[j]);
+template <int N, bool AXIS0>
+__global__ void __launch_bounds__(line_threads<N>(AXIS0)) k_adj_line(RowLayout L, LineArgs A) {
+  constexpr int NT = line_threads<N>(AXIS0);
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double2* sv = reinterpret_cast<double2*>(smraw);   // v: AXIS0 [line][N+1], else [j][thread]
+  double2* st = sv + NT * (N + 1);                   // AXIS0: the lam tile, later fft(x u)
+  const int tid = threadIdx.x;
+  const long long nlines = L.nrows * (L.nx / N), groups = (nlines + NT - 1) / NT;
+  long long stride = 1;
+  for (int a = 0; a < A.axis; ++a) stride *= N;
+  const double tp = 2.0 * M_PI / A.Llen;
+  double dot = 0.0;
+  for (long long g = blockIdx.x; g < groups; g += gridDim.x) {
+    const long long t = g * NT + tid;
+    const bool ok = t < nlines;
+    const int cnt = (int)min((long long)NT, nlines - g * NT);      // lines of this group
+    const long long g0 = g * NT * N;                               // AXIS0: the group's first value
+    long long base = 0, row = 0;
+    if (AXIS0) {
+      __syncthreads();   // the previous group's tiles are done with
+      for (int e = tid; e < cnt * N; e += NT) {
+        cp_async<16>(st + (e / N) * (N + 1) + e % N, A.lam + g0 + e, true);
+        if (A.F) cp_async<16>(sv + (e / N) * (N + 1) + e % N, A.F + g0 + e, true);
       }
+      cp_async_wait_all();
+      __syncthreads();
+      if (ok) row = t / (L.nx / N);
+    } else if (ok) {
+      const long long per = L.nx / N, q = t % per;
+      row = t / per;
+      base = row * L.nx + q / stride * stride * N + q % stride;
+    }
+    double2* v = AXIS0 ? sv + tid * (N + 1) : sv + tid;
+    constexpr int VS = AXIS0 ? 1 : NT;                             // distance of the values of v
+    double2 x[N];
+    if (ok) {
+      if (A.F) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) x[j] = AXIS0 ? v[j] : A.F[base + j * stride];
+        fft<N, true>(x);
+#pragma unroll
+        for (int j = 0; j < N; ++j) v[j * VS] = x[j];
+        if (!AXIS0 && A.Y2) {
+#pragma unroll
+          for (int j = 0; j < N; ++j) A.Y2[base + j * stride] = x[j];
+        }
+      }
+      if (!AXIS0 && A.Y1) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) x[j] = A.lam[base + j * stride];
+        fft<N, true>(x);
+#pragma unroll
+        for (int j = 0; j < N; ++j) A.Y1[base + j * stride] = x[j];
+      }
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+        const double2 u = AXIS0 ? st[tid * (N + 1) + j] : A.lam[base + j * stride];
+        const double dk = tp * kappa_first(j, N);
+        x[j] = make_double2(-dk * u.y, dk * u.x);   // i dk lam
+      }
+      fft<N, true>(x);
+      double s = 0.0;
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+        const double xc = (-A.Llen / 2 + A.Llen * j / N) / N;
+        x[j] = xc * x[j];
+        if (A.F) s += x[j].x * v[j * VS].x + x[j].y * v[j * VS].y;
+      }
+      if (A.F) dot -= A.scale * row_weight(L, row, A.half) * s;
+      if (A.out) {
+        fft<N, false>(x);
+        if (AXIS0) {
+#pragma unroll
+          for (int j = 0; j < N; ++j) st[tid * (N + 1) + j] = x[j];
+        } else {
+#pragma unroll
+          for (int j = 0; j < N; ++j) {
+            double2 o = A.out[base + j * stride];
+            o.x += A.coef * x[j].x;
+            o.y += A.coef * x[j].y;
+            A.out[base + j * stride] = o;
+          }
+        }
+      }
+    }
+    if (AXIS0 && A.out) {
+      __syncthreads();
+      for (int e = tid; e < cnt * N; e += NT) {
+        const double2 w = st[(e / N) * (N + 1) + e % N];
+        double2 o = A.out[g0 + e];
+        o.x += A.coef * w.x;
+        o.y += A.coef * w.y;
+        A.out[g0 + e] = o;
+      }
+    }
   }
-  for (int q = 0; q < 6; ++q) red[q][threadIdx.x] = s[q];
-  __syncthreads();
-  for (int k = kDotThreads / 2; k > 0; k >>= 1) {
-    if (threadIdx.x < k)
-      for (int q = 0; q < 6; ++q) red[q][threadIdx.x] += red[q][threadIdx.x + k];
-    __syncthreads();
-  }
-  if (threadIdx.x < 6) acc[(long long)(slot0 + threadIdx.x) * gridDim.x + blockIdx.x] += scale * red[threadIdx.x][0];
+  if (A.F) block_add(dot, A.acc, A.slot);
 }
 
-// out = (in + C in) / 2 on the full layout, C the real-density mirror
-// F^l_{mn}[k] -> (-1)^(m-n) conj F^l_{-m,-n}[-k].
-__global__ void k_sym_full(int lmax, int N, int ndim, long long nx, const double2* __restrict__ in,
-                           double2* __restrict__ out) {
-  const int D = 2 * lmax + 1;
-  const long long Dfull = (long long)D * D * (lmax + 1);
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= Dfull * nx) return;
-  const long long fi = t % Dfull, w = t / Dfull;
-  const int m = (int)(fi % D) - lmax, n = (int)((fi / D) % D) - lmax, l = (int)(fi / ((long long)D * D));
-  long long wm = 0, mul = 1, ww = w;
-  for (int a = 0; a < ndim; ++a) {
-    const int k = (int)(ww % N);
-    ww /= N;
-    wm += mul * ((N - k) % N);
-    mul *= N;
+// The gradient of gyro_i: Re<lam, -D_i M_j M_k F> from a = ifft_j ifft_k lam and
+// b = ifft_j ifft_k F, per point d_i x_j x_k Im(conj(a) b) / N^2.  Y1, Y2 hold
+// the inverse transforms along one of the two axes (oaxis), the lines run
+// along the other (axis); daxis = i.
+template <int N, bool AXIS0>
+__global__ void __launch_bounds__(line_threads<N>(AXIS0)) k_gyro_dot(RowLayout L, const double2* __restrict__ Y1,
+                                                                     const double2* __restrict__ Y2, int axis, int oaxis,
+                                                                     int daxis, double scale, double Llen, int half,
+                                                                     double* __restrict__ acc, int slot) {
+  constexpr int NT = line_threads<N>(AXIS0);
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double2* sa = reinterpret_cast<double2*>(smraw);
+  double2* sb = sa + NT * (N + 1);                    // AXIS0 only
+  const int tid = threadIdx.x;
+  const long long per = L.nx / N, nlines = L.nrows * per, groups = (nlines + NT - 1) / NT;
+  long long stride = 1, os = 1, ds = 1;
+  for (int a = 0; a < axis; ++a) stride *= N;
+  for (int a = 0; a < oaxis; ++a) os *= N;
+  for (int a = 0; a < daxis; ++a) ds *= N;
+  double dot = 0.0;
+  for (long long g = blockIdx.x; g < groups; g += gridDim.x) {
+    const long long t = g * NT + tid;
+    const int cnt = (int)min((long long)NT, nlines - g * NT);
+    const long long g0 = g * NT * N;
+    if (AXIS0) {
+      __syncthreads();
+      for (int e = tid; e < cnt * N; e += NT) {
+        cp_async<16>(sa + (e / N) * (N + 1) + e % N, Y1 + g0 + e, true);
+        cp_async<16>(sb + (e / N) * (N + 1) + e % N, Y2 + g0 + e, true);
+      }
+      cp_async_wait_all();
+      __syncthreads();
+    }
+    if (t >= nlines) continue;
+    const long long row = t / per, q = t % per;
+    const long long w = q / stride * stride * N + q % stride, base = row * L.nx + w;   // the line's first point
+    double2* a = AXIS0 ? sa + tid * (N + 1) : sa + tid;
+    constexpr int VS = AXIS0 ? 1 : NT;
+    double2 x[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) x[j] = AXIS0 ? a[j] : Y1[base + j * stride];
+    fft<N, true>(x);
+#pragma unroll
+    for (int j = 0; j < N; ++j) a[j * VS] = x[j];
+#pragma unroll
+    for (int j = 0; j < N; ++j) x[j] = AXIS0 ? sb[tid * (N + 1) + j] : Y2[base + j * stride];
+    fft<N, true>(x);
+    double s = 0.0;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const double xc = -Llen / 2 + Llen * j / N;
+      const double2 u = a[j * VS];
+      s += xc * (u.x * x[j].y - u.y * x[j].x);
+    }
+    const double dk = 2.0 * M_PI / Llen * kappa_first((int)(w / ds % N), N);
+    const double xo = -Llen / 2 + Llen * (double)(w / os % N) / N;
+    dot += scale * row_weight(L, row, half) * dk * xo / ((double)N * N) * s;
   }
-  const long long fm = (-m + lmax) + (long long)D * (-n + lmax) + (long long)D * D * l;
-  const double2 a = in[t], b = in[fm + Dfull * wm];
-  const double sg = ((m - n) & 1) ? -1.0 : 1.0;
-  out[t] = make_double2(0.5 * (a.x + sg * b.x), 0.5 * (a.y - sg * b.y));
+  block_add(dot, acc, slot);
 }
 
 template <int N>
-int axis_md_launch(hp_plan* p, const double2* in, double2* out, int axis, double coef, cudaStream_t s) {
-  const long long nl = p->nrows * (p->nx / N);
+int adj_line_launch(hp_plan* p, const LineArgs& A, cudaStream_t s) {
   ProfScope _ps(p, "adj.axis", s);
-  k_axis_md<N><<<(unsigned)((nl + 127) / 128), 128, 0, s>>>(p->layout(), in, out, axis, coef, p->model.L);
-  HP_CUDA_TRY(cudaGetLastError());
-  return HP_OK;
+  auto go = [&](auto kern, bool a0) -> int {
+    HP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)line_smem<N>(a0)));
+    kern<<<kDotBlocks, line_threads<N>(a0), line_smem<N>(a0), s>>>(p->layout(), A);
+    HP_CUDA_TRY(cudaGetLastError());
+    return HP_OK;
+  };
+  return A.axis == 0 ? go(k_adj_line<N, true>, true) : go(k_adj_line<N, false>, false);
 }
 
 template <int N>
-int line_dm_launch(hp_plan* p, const double2* in, double2* out, int axis, int daxis, double coef, int acc,
-                   cudaStream_t s) {
-  const long long nl = p->nrows * (p->nx / N);
+int gyro_dot_launch(hp_plan* p, const double2* Y1, const double2* Y2, int axis, int oaxis, int daxis, double scale,
+                    double* acc, int slot, cudaStream_t s) {
   ProfScope _ps(p, "adj.axis", s);
-  k_line_dm<N><<<(unsigned)((nl + 127) / 128), 128, 0, s>>>(p->layout(), in, out, axis, daxis, coef, p->model.L, acc);
-  HP_CUDA_TRY(cudaGetLastError());
-  return HP_OK;
+  const int half = p->symmetry == HP_REAL;
+  auto go = [&](auto kern, bool a0) -> int {
+    HP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)line_smem<N>(a0)));
+    kern<<<kDotBlocks, line_threads<N>(a0), line_smem<N>(a0), s>>>(p->layout(), Y1, Y2, axis, oaxis, daxis, scale,
+                                                                   p->model.L, half, acc, slot);
+    HP_CUDA_TRY(cudaGetLastError());
+    return HP_OK;
+  };
+  return axis == 0 ? go(k_gyro_dot<N, true>, true) : go(k_gyro_dot<N, false>, false);
 }
 
-// out = coef D_daxis M_axis in (acc: out += ...)
-int line_dm(hp_plan* p, const double2* in, double2* out, int axis, int daxis, double coef, int acc,
-            cudaStream_t s) {
+// every omega grid size
+int adj_line(hp_plan* p, const LineArgs& A, cudaStream_t s) {
   switch (p->N) {
-#define X(n) case n: return line_dm_launch<n>(p, in, out, axis, daxis, coef, acc, s);
+#define X(n) case n: return adj_line_launch<n>(p, A, s);
     HP_FOR_EACH_N(X)
 #undef X
     default:
@@ -262,97 +287,78 @@ int line_dm(hp_plan* p, const double2* in, double2* out, int axis, int daxis, do
   }
 }
 
-int axis_md(hp_plan* p, const double2* in, double2* out, int axis, double coef, cudaStream_t s) {
+int gyro_dot(hp_plan* p, const double2* Y1, const double2* Y2, int axis, int oaxis, int daxis, double scale, double* acc,
+             int slot, cudaStream_t s) {
   switch (p->N) {
-#define X(n) case n: return axis_md_launch<n>(p, in, out, axis, coef, s);
+#define X(n) case n: return gyro_dot_launch<n>(p, Y1, Y2, axis, oaxis, daxis, scale, acc, slot, s);
     HP_FOR_EACH_N(X)
 #undef X
     default:
       hp_set_error("omega grid size 2Bx not supported (even, 4..64)");
       return HP_ERR_UNSUPPORTED;
   }
-}
-
-// out = (add ? lam : 0) + a * A^H lam   (internal layout, FP64 buffers)
-int adjoint_apply(hp_plan* p, const double2* lam, double2* out, double a, int add, cudaStream_t s) {
-  const DerivParams base = hp_model_params(p);
-  DerivParams q = base;
-  for (int i = 0; i < 3; ++i) q.b[i] = 0.0;
-  for (int i = 0; i < 9; ++i) q.G[i] = -base.G[i];
-  int st = HP_OK;
-  const size_t ib = 16 * (size_t)p->nrows * p->nx;
-  double2* t = (double2*)p->ws_get("adj.t", ib, &st);
-  if (st) return st;
-  double2* d1 = (double2*)p->ws_get("adj.d1", ib, &st);
-  if (st) return st;
-  const long long n = p->nrows * p->nx;
-  const unsigned g = (unsigned)((n + 255) / 256);
-  {
-    ProfScope _ps(p, "adj.weight", s);
-    k_row_unweight<<<g, 256, 0, s>>>(p->layout(), lam, t);
-    HP_CUDA_TRY(cudaGetLastError());
-  }
-  ADJ_CHECK(hp_derivative_eval_prm(p, q, t, nullptr, 1.0, d1, nullptr, 0.0, s));
-  {
-    ProfScope _ps(p, "adj.weight", s);
-    k_adj_combine<<<g, 256, 0, s>>>(p->layout(), lam, d1, out, a, add);
-    HP_CUDA_TRY(cudaGetLastError());
-  }
-  for (int i = 0; i < p->ndim; ++i)
-    if (base.b[i] != 0.0) ADJ_CHECK(axis_md(p, lam, out, i, -a * base.b[i], s));
-  return HP_OK;
 }
 
 // Gradient slots: b[0..2], gyro[3..5], gscale[6..8], G pairs [9..14]
 // ((0,0),(0,1),(0,2),(1,1),(1,2),(2,2)).
 constexpr int kSlots = 15;
 
-// acc += dt * Re<lam, dA/dtheta F> for every parameter theta.  The terms of
-// the derivative are linear in their parameters, so dA/dtheta F is the term
-// itself with unit coefficient, each formed by the passes it needs alone:
-//   damping   dA/db_i F    =  D_i M_i F            (one line pass)
-//   gyroscope dA/dgyro_i F = -D_i M_j M_k F        (two line passes; j, k the other axes)
-//   gravity   dA/dgs_i F   =  the gravity pass with component i alone
-// (the forms of the plane pass's Y0, Y1, Y2 products and the axis-3 pass).
-int grad_terms(hp_plan* p, const double2* lam, const double2* F, double dt, double* acc, cudaStream_t s) {
+// out = (add ? lam : 0) + a * A^H lam   (internal layout, FP64 buffers), and
+// with F also acc += dt * Re<lam, dA/dtheta F> for every parameter theta.  The
+// terms of the derivative are linear in their parameters, so dA/dtheta F is
+// the term itself with unit coefficient:
+//   damping   dA/db_i F    =  D_i M_i F,  gyroscope dA/dgyro_i F = -D_i M_j M_k F,
+//   gravity   dA/dgs_i F   = -D_i Grav_i F,  noise dA/dG_ij F = c_ij F.
+// The bracket of A^H is one derivative evaluation that adds itself to lam (its
+// gravity taps are those of W Grav W^-1); each axis then takes one pass
+// (k_adj_line) for its damping adjoint and damping gradient.  Dots of fields
+// kept on the grid along one axis (Y1, Y2) give the gyroscopic gradients.
+int adjoint_apply(hp_plan* p, const double2* lam, const double2* F, double2* out, double a, int add, double dt,
+                  double* acc, cudaStream_t s) {
   const DerivParams base = hp_model_params(p);
+  DerivParams q = base;
+  for (int i = 0; i < 3; ++i) q.b[i] = 0.0;
+  for (int i = 0; i < 9; ++i) q.G[i] = -base.G[i];
   int st = HP_OK;
-  const size_t ib = 16 * (size_t)p->nrows * p->nx;
-  double2* y = (double2*)p->ws_get("adj.y", ib, &st);
+  bool have = false;
+  for (auto& kv : p->ws) if (kv.first == "adj.taps" && kv.second.p) have = true;
+  void* taps = p->ws_get("adj.taps", (p->precision == HP_FP64 ? sizeof(double) : sizeof(float)) * 9 * p->nrows, &st);
   if (st) return st;
-  const int half = p->symmetry == HP_REAL;
-  auto dot = [&](int slot) -> int {
-    ProfScope _ps(p, "adj.dot", s);
-    k_dot<<<kDotBlocks, kDotThreads, 0, s>>>(p->layout(), lam, y, acc, slot, dt, half);
-    HP_CUDA_TRY(cudaGetLastError());
-    return HP_OK;
-  };
-  for (int i = 0; i < p->ndim; ++i) {
-    ADJ_CHECK(line_dm(p, F, y, i, i, 1.0, 0, s));
-    ADJ_CHECK(dot(i));
-  }
-  if (p->ndim == 3) {
-    double2* t = (double2*)p->ws_get("adj.t", ib, &st);
+  if (!have) ADJ_CHECK(hp_adjoint_gravity_taps(p, taps, s));
+  q.taps = taps;
+  const size_t ib = 16 * (size_t)p->nrows * p->nx;
+  double2 *y1 = nullptr, *y2 = nullptr;
+  if (F && p->ndim == 3) {
+    y1 = (double2*)p->ws_get("adj.t", ib, &st);
     if (st) return st;
-    for (int i = 0; i < 3; ++i) {
-      const int j = (i + 1) % 3, k = (i + 2) % 3;
-      ADJ_CHECK(line_dm(p, F, t, j, -1, 1.0, 0, s));
-      ADJ_CHECK(line_dm(p, t, y, k, i, -1.0, 0, s));
-      ADJ_CHECK(dot(3 + i));
+    y2 = (double2*)p->ws_get("adj.y", ib, &st);
+    if (st) return st;
+  }
+  ADJ_CHECK(hp_derivative_eval_prm(p, q, lam, add ? lam : nullptr, -a, out, nullptr, 0.0, s));
+  if (F) ADJ_CHECK(hp_gravity_noise_dots64(p, F, lam, acc, kDotBlocks, 6, dt, s));
+  for (int i = p->ndim - 1; i >= 0; --i) {
+    LineArgs A{};
+    A.lam = lam;
+    A.F = F;
+    A.out = base.b[i] != 0.0 ? out : nullptr;
+    A.Y1 = i > 0 ? y1 : nullptr;
+    A.Y2 = i > 0 ? y2 : nullptr;
+    A.axis = i;
+    A.coef = -a * base.b[i];
+    A.scale = dt;
+    A.Llen = base.L;
+    A.half = p->symmetry == HP_REAL;
+    A.slot = i;
+    A.acc = acc;
+    if (F || A.out) ADJ_CHECK(adj_line(p, A, s));
+    if (!y1) continue;
+    if (i == 2) {   // on the grid along axis 2: gyro_0 along axis 1, gyro_1 along axis 0
+      ADJ_CHECK(gyro_dot(p, y1, y2, 1, 2, 0, dt, acc, 3, s));
+      ADJ_CHECK(gyro_dot(p, y1, y2, 0, 2, 1, dt, acc, 4, s));
+    } else if (i == 1) {
+      ADJ_CHECK(gyro_dot(p, y1, y2, 0, 1, 2, dt, acc, 5, s));
     }
   }
-  for (int i = 0; i < p->ndim; ++i) {
-    DerivParams z = base;
-    for (int a = 0; a < 3; ++a) { z.b[a] = 0; z.gyro[a] = 0; z.gs[a] = 0; }
-    for (int a = 0; a < 9; ++a) z.G[a] = 0;
-    z.lie = 0;
-    z.gs[i] = 1.0;
-    ADJ_CHECK(hp_gravity_noise_eval64(p, z, F, y, s));
-    ADJ_CHECK(dot(6 + i));
-  }
-  ProfScope _ps(p, "adj.dot", s);
-  k_dot_noise<<<kDotBlocks, kDotThreads, 0, s>>>(p->layout(), lam, F, acc, 9, dt, half, p->model.L);
-  HP_CUDA_TRY(cudaGetLastError());
   return HP_OK;
 }
 
@@ -363,27 +369,16 @@ int check_mem(int mem) {
 
 // full-layout (mem) -> internal FP64, symmetrised for HP_REAL plans
 int load_full(hp_plan* p, const double* src, int mem, double2* dst, cudaStream_t s) {
-  int st = HP_OK;
-  const size_t fb = 16 * (size_t)p->n_full();
-  double2* a = (double2*)p->ws_get("adj.full_a", fb, &st);
-  if (st) return st;
   const double2* in = (const double2*)src;
   if (mem == HP_HOST) {
+    int st = HP_OK;
+    const size_t fb = 16 * (size_t)p->n_full();
+    double2* a = (double2*)p->ws_get("adj.full_a", fb, &st);
+    if (st) return st;
     HP_CUDA_TRY(cudaMemcpyAsync(a, src, fb, cudaMemcpyHostToDevice, s));
     in = a;
   }
-  if (p->symmetry == HP_REAL) {
-    double2* b = (double2*)p->ws_get("adj.full_b", fb, &st);
-    if (st) return st;
-    const long long n = p->n_full();
-    {
-      ProfScope _ps(p, "layout", s);
-      k_sym_full<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(p->lmax, p->N, p->ndim, p->nx, in, b);
-      HP_CUDA_TRY(cudaGetLastError());
-    }
-    in = b;
-  }
-  return hp_full_to_internal(p, in, dst, s);
+  return p->symmetry == HP_REAL ? hp_full_to_internal_sym(p, in, dst, s) : hp_full_to_internal(p, in, dst, s);
 }
 
 int store_full(hp_plan* p, const double2* src, double* dst, int mem, cudaStream_t s) {
@@ -427,7 +422,7 @@ extern "C" int hp_pendulum_derivative_adjoint(hp_plan* p, const double* lam, dou
     }
     ADJ_CHECK(hp_full_to_internal(p, in, li, s));
   }
-  ADJ_CHECK(adjoint_apply(p, li, lo, 1.0, 0, s));
+  ADJ_CHECK(adjoint_apply(p, li, nullptr, lo, 1.0, 0, 0.0, nullptr, s));
   ADJ_CHECK(store_full(p, lo, out, mem, s));
   HP_CUDA_TRY(cudaStreamSynchronize(s));
   return HP_OK;
@@ -490,8 +485,7 @@ extern "C" int hp_pendulum_adjoint(hp_plan* p, const double* F0, const double* l
     for (int j = 1; j < len; ++j)
       ADJ_CHECK(hp_derivative_eval(p, state(seg, j - 1), state(seg, j - 1), dt, state(seg, j), nullptr, 0.0, s));
     for (int j = len - 1; j >= 0; --j) {
-      ADJ_CHECK(grad_terms(p, la, state(seg, j), dt, acc, s));
-      ADJ_CHECK(adjoint_apply(p, la, lb, dt, 1, s));
+      ADJ_CHECK(adjoint_apply(p, la, state(seg, j), lb, dt, 1, dt, acc, s));
       std::swap(la, lb);
     }
   }

@@ -173,6 +173,7 @@ struct DerivParams {
   double lie;
   double gs[3];
   double mr[3][3][2];  // MR_i^1_{0 n2}: [n2+1][i][re, im]
+  const void* taps = nullptr;   // gravity tap weights in the compute precision (null: the plan's)
 };
 // Persistent batched plane pass (deriv.cu): between hp_plane_collect_begin and
 // _end, the plane passes of 3-D derivative evaluations are recorded as jobs
@@ -210,10 +211,13 @@ DerivParams hp_model_params(const hp_plan* p);
 int hp_derivative_eval_prm(hp_plan* p, const DerivParams& prm, const double2* Feval, const double2* F0,
                            double a, double2* out, double2* acc, double bacc, cudaStream_t s,
                            const void* fgrid = nullptr, const void* fev32 = nullptr, void* out32 = nullptr);
-// The gravity and noise terms of the derivative alone (the pointwise-in-omega
-// pass), in FP64 whatever the plan's precision: out = noise F + gravity F
-// ([row][omega] layout, FP64 in and out).
-int hp_gravity_noise_eval64(hp_plan* p, const DerivParams& prm, const double2* F, double2* out, cudaStream_t s);
+// Gradient dot products of the gravity and noise terms in FP64 (one pass over F
+// and lam): acc[(slot + i) * nblocks + block] += scale * Re<lam, -D_i Grav_i F>,
+// i < 3, and acc[(slot + 3 + q) * nblocks + block] += scale * Re<lam, c_ij F> for
+// the pairs q of (0,0), (0,1), (0,2), (1,1), (1,2), (2,2); rows with m > 0 count
+// twice in HP_REAL plans.  At most nblocks blocks run.
+int hp_gravity_noise_dots64(hp_plan* p, const double2* F, const double2* lam, double* acc, int nblocks, int slot,
+                            double scale, cudaStream_t s);
 int hp_derivative_eval(hp_plan* p, const double2* Feval, const double2* F0, double a,
                        double2* out, double2* acc, double bacc, cudaStream_t s,
                        const void* fgrid = nullptr, const void* fev32 = nullptr, void* out32 = nullptr);
