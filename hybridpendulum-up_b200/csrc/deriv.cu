@@ -251,9 +251,27 @@ template <typename T> static constexpr int local_w() { return sizeof(T) == 8 ? 1
 
 // --------------------------------------------------- pass C: plane pass ----
 
-template <typename T> struct PlaneCfg;
+template <typename T> struct PlaneCfg;   // MINB: blocks per SM of the persistent batched pass
 template <> struct PlaneCfg<double> { static constexpr int C = 1; static constexpr int NT = 128; static constexpr int MINB = 2; };
 template <> struct PlaneCfg<float> { static constexpr int C = 2; static constexpr int NT = 256; static constexpr int MINB = 2; };
+
+// Resident blocks per SM that the registers are held to.  The pass waits for
+// its own barriers and FP64 chains more than for anything it could compute, so
+// more blocks pay even where a few registers spill; shared memory (C + 2 F
+// planes, C each of P and Y) sets the limit from N = 22 on.  B = 10, ms per pass
+// with two blocks / these: FP64 N = 16 0.234 / 0.132, 24 0.648 / 0.453, 30 1.153
+// / 0.979; FP32 N = 16 0.128 / 0.089, 24 0.343 / 0.287, 30 0.646 / 0.601.  FP32 at
+// N = 32: three blocks 0.594, two 0.573; FP64 at N = 20: five 0.323, four 0.314.
+// Not kept: runs of consecutive n sharing their physical planes with every FFT
+// on a lane pair (half the inverse FFTs, but 0.5 KB of spills: FP32 1.85 -> 2.24
+// at B = 15, 32^3; FP64 unchanged).
+template <int N, typename T, bool HAS_P3> constexpr int plane_minb() {
+  if (sizeof(T) == 8) {
+    if (N <= 16 && !HAS_P3) return 4;   // small 2-D grids: latency of one block counts
+    return N <= 12 ? 8 : N <= 16 ? 5 : N <= 24 ? 4 : N <= 30 ? 3 : 2;
+  }
+  return N <= 24 ? 4 : N <= 30 ? 3 : 2;
+}
 
 __device__ __forceinline__ long long row_of(const RowLayout& L, int l, int m, int n) {
   const int am = abs(m), an = abs(n);
@@ -263,8 +281,9 @@ __device__ __forceinline__ long long row_of(const RowLayout& L, int l, int m, in
 // smem planes (stride PS = N*(N+1)):
 //   [0, C+2)           F~ rows n0-1 .. n0+C     (physical after the inverse FFTs)
 //   [C+2, 2C+2)        P~ rows n0 .. n0+C-1     (ndim = 3)
-//   [2C+2, 3C+2)       A  = FFT2(Y0) + D_2 FFT2(Y2), then FFT_1
-//   [3C+2, 4C+2)       Y1' = FFT_2(Y1), then D_1 FFT_1
+//   [2C+2, 3C+2)       Y1' = FFT_2(Y1), then D_1 FFT_1
+// A = FFT2(Y0) + D_2 FFT2(Y2), then FFT_1, overwrites the plane of F~ that only
+// its own Y0 reads: row n0-1 for the tile's first row, n0+2 for its second.
 // One tile (tl) on one k3 plane: the body of k_plane, also run by the
 // persistent batched plane pass (k_plane_batch) for tiles of many members.
 template <int N, typename T, bool HAS_P3, typename TIN>
@@ -280,8 +299,8 @@ __device__ __forceinline__ void plane_body(const RowLayout& L, const PlaneTile t
   C* sm = reinterpret_cast<C*>(smraw);
   C* sF = sm;
   C* sP = sm + (CT + 2) * PS;
-  C* sA = sm + (CT + 2 + NP) * PS;
-  C* sY = sm + (CT + 2 + NP + CT) * PS;
+  C* sY = sm + (CT + 2 + NP) * PS;
+  auto plane_A = [&](int c) -> C* { return sF + (c == 0 ? 0 : (CT + 1) * PS); };
 
   const long long pbase = (long long)k3 * N * N;  // plane offset inside a row
   const int tid = threadIdx.x, nth = blockDim.x;
@@ -459,7 +478,7 @@ __device__ __forceinline__ void plane_body(const RowLayout& L, const PlaneTile t
       }
       fft_lane_pair<H, false>(x, h);
 #pragma unroll
-      for (int k = 0; k < H; ++k) sA[c * PS + (h * H + k) * (N + 1) + j1] = x[k];
+      for (int k = 0; k < H; ++k) plane_A(c)[(h * H + k) * (N + 1) + j1] = x[k];
       // Y2 = b2 x2 F~ - g2 x1 P~  -> FFT_2 -> times D_2 = i d2(k2), added to A
 #pragma unroll
       for (int j = 0; j < H; ++j) {
@@ -475,7 +494,7 @@ __device__ __forceinline__ void plane_body(const RowLayout& L, const PlaneTile t
       for (int k = 0; k < H; ++k) {
         const int k2 = h * H + k;
         const T dk = tp * (T)kappa_first(k2, N);
-        C* dst = sA + c * PS + k2 * (N + 1) + j1;
+        C* dst = plane_A(c) + k2 * (N + 1) + j1;
         C v = *dst;
         v.x -= dk * x[k].y;
         v.y += dk * x[k].x;
@@ -506,7 +525,7 @@ __device__ __forceinline__ void plane_body(const RowLayout& L, const PlaneTile t
     const int kind = it / (tl.cnt * N);
     const int c = (it / N) % tl.cnt;
     const int k2 = it % N;
-    C* pl = (kind == 0 ? sA : sY) + c * PS + k2 * (N + 1);
+    C* pl = (kind == 0 ? plane_A(c) : sY + c * PS) + k2 * (N + 1);
     C x[H];
 #pragma unroll
     for (int j = 0; j < H; ++j) x[j] = pl[2 * j + h];
@@ -552,7 +571,7 @@ __device__ __forceinline__ void plane_body(const RowLayout& L, const PlaneTile t
         const int e = e0 + u * nth;
         if (e >= tot) continue;
         const int c = e / (N * N), q = e % (N * N), k1 = q % N, k2 = q / N;
-        const C s = sA[c * PS + k2 * (N + 1) + k1] + sY[c * PS + k2 * (N + 1) + k1];
+        const C s = plane_A(c)[k2 * (N + 1) + k1] + sY[c * PS + k2 * (N + 1) + k1];
         const double dx = (double)s.x + (double)g[u].x, dy = (double)s.y + (double)g[u].y;
         double2 o = f0[u];
         o.x += a * dx;
@@ -573,7 +592,7 @@ __device__ __forceinline__ void plane_body(const RowLayout& L, const PlaneTile t
 }
 
 template <int N, typename T, bool HAS_P3, typename TIN>
-__global__ void __launch_bounds__(PlaneCfg<T>::NT, PlaneCfg<T>::MINB) k_plane(RowLayout L, const PlaneTile* __restrict__ tiles,
+__global__ void __launch_bounds__(PlaneCfg<T>::NT, (plane_minb<N, T, HAS_P3>())) k_plane(RowLayout L, const PlaneTile* __restrict__ tiles,
                                                   const c2<TIN>* __restrict__ Fev,
                                                   const c2<T>* __restrict__ P3,
                                                   const c2<T>* __restrict__ Gl,
@@ -650,7 +669,7 @@ bool hp_plane_collecting() { return g_collect[0] || g_collect[1]; }
 
 template <typename T> static size_t plane_smem_p3(int N) {
   constexpr int C = PlaneCfg<T>::C;
-  return (size_t)((C + 2) + C + 2 * C) * N * (N + 1) * sizeof(c2<T>);
+  return (size_t)((C + 2) + C + C) * N * (N + 1) * sizeof(c2<T>);
 }
 size_t hp_plane_batch_smem(int precision, int Nmax) {
   return precision == HP_FP64 ? plane_smem_p3<double>(Nmax) : plane_smem_p3<float>(Nmax);
@@ -696,7 +715,7 @@ int hp_plane_batch_launch(int precision, const std::vector<PlaneJob>& jobs, cons
 // ------------------------------------------------------------ launcher ----
 template <typename T> static size_t plane_smem(int N, bool p3) {
   const int C = PlaneCfg<T>::C;
-  const int planes = (C + 2) + (p3 ? C : 0) + 2 * C;
+  const int planes = (C + 2) + (p3 ? C : 0) + C;
   return (size_t)planes * N * (N + 1) * sizeof(c2<T>);
 }
 
