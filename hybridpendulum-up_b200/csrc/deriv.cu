@@ -85,44 +85,63 @@ __global__ void __launch_bounds__(128) k_axis3(RowLayout L, const c2<TIN>* __res
 // warp-uniform and reads shared memory only.  Per omega point the model part
 // of the weights folds into nu[n2] = -i sum_i D_i gs_i MR_i^1_{0 n2}, so
 //   G = noise F + sum_{n2} nu[n2] sum_{l1} w(l1, n2) F^{l1}_{m, n-n2}.
+// Bound by the shared-memory pipe: 9 source values per output, and the row's
+// weights and sources, which come as whole vectors from tables built with the
+// plan (one by one, with the sources recomputed by every block, the pass took
+// 0.49 ms at B = 15, 32^3, FP32 and 12.6 us at B = 8, 16 x 16; now 0.42 and 10.9).
 template <typename T> __host__ __device__ constexpr size_t local_tile_bytes(int rmax, int W) {
   return ((size_t)rmax * W * sizeof(c2<T>) + 15) / 16 * 16;
 }
 
+// The nine weights and nine sources of row r of an m group, read 16 bytes
+// (weights) and 8 bytes (sources) at a time.
+template <typename T> struct Taps {
+  T w[kTapStride];
+  short src[kTapStride];
+  __device__ __forceinline__ void load(const T* sw, const short* ssrc, int r) {
+    struct alignas(16) V { T v[16 / sizeof(T)]; };
+#pragma unroll
+    for (int k = 0; k < kTapStride; k += 16 / (int)sizeof(T))
+      *reinterpret_cast<V*>(w + k) = *reinterpret_cast<const V*>(sw + r * kTapStride + k);
+#pragma unroll
+    for (int k = 0; k < kTapStride; k += 4)
+      *reinterpret_cast<short4*>(src + k) = *reinterpret_cast<const short4*>(ssrc + r * kTapStride + k);
+  }
+};
+
 template <typename T, int W, int NDIM, typename TIN>
 __global__ void __launch_bounds__(256) k_local(RowLayout L, const c2<TIN>* __restrict__ F,
                                                c2<T>* __restrict__ G, const T* __restrict__ tap_wr,
-                                               const c2<T>* __restrict__ Gx, const c2<T>* __restrict__ sdk,
-                                               DerivParams prm, int cpb) {
+                                               const short* __restrict__ tap_src, const c2<T>* __restrict__ Gx,
+                                               const c2<T>* __restrict__ sdk, DerivParams prm, int cpb) {
   using C = c2<T>;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int D = 2 * L.lmax + 1;
   const int rmax = (L.lmax + 1) * (L.lmax + 1);
   C* tile = reinterpret_cast<C*>(smraw);                                          // [R][W]
-  T* sw = reinterpret_cast<T*>(smraw + local_tile_bytes<T>(rmax, W));             // [R][9]
-  int* sseg = reinterpret_cast<int*>(smraw + local_tile_bytes<T>(rmax, W) +
-                                     ((size_t)rmax * 9 * sizeof(T) + 15) / 16 * 16);  // [D]
-  short* ssrc = reinterpret_cast<short*>(sseg + (D + 3) / 4 * 4);                 // [R][9]
+  T* sw = reinterpret_cast<T*>(smraw + local_tile_bytes<T>(rmax, W));             // [R][kTapStride]
+  short* ssrc = reinterpret_cast<short*>(sw + (size_t)rmax * kTapStride);         // [R][kTapStride]
+  int* sseg = reinterpret_cast<int*>(ssrc + (size_t)rmax * kTapStride);           // [D]
   const int m = (int)blockIdx.y + L.m_lo;
   const int r0 = L.seg[(m - L.m_lo) * D];
   const int r1 = (m + 1 <= L.lmax) ? L.seg[(m + 1 - L.m_lo) * D] : (int)L.nrows;
   const int R = r1 - r0;
   const int tid = threadIdx.x, nth = blockDim.x;
   // per block, once for its cpb omega chunks: the group's tap weights and tap
-  // sources
-  for (int e = tid; e < R * 9; e += nth) sw[e] = tap_wr[(size_t)r0 * 9 + e];
-  for (int e = tid; e < D; e += nth) sseg[e] = L.seg[(m - L.m_lo) * D + e] - r0;
-  // tap t = (l1 - l + 1) * 3 + (n2 + 1) of row r reads group row ssrc[r][t]
-  // (row 0 where the tap has no weight), so the tap loop below has no branches
-  const int am = abs(m), lmax = L.lmax;
-  for (int e = tid; e < R * 9; e += nth) {
-    const char4 q = L.rows[r0 + e / 9];
-    const int t = e % 9, l1 = q.x + t / 3 - 1, n1 = q.z - (t % 3 - 1), an1 = abs(n1);
-    int src = 0;
-    if (l1 >= 0 && l1 <= lmax && am <= l1 && an1 <= l1)
-      src = L.seg[(m - L.m_lo) * D + n1 + lmax] - r0 + l1 - (am > an1 ? am : an1);
-    ssrc[e] = (short)src;
+  // sources, straight copies of the tables (the tap t = (l1 - l + 1) * 3 +
+  // (n2 + 1) of row r reads group row src[r][t], row 0 where it has no weight,
+  // so the tap loop below has no branches)
+  {
+    constexpr int EP = 16 / (int)sizeof(T);
+    const T* tw = tap_wr + (size_t)r0 * kTapStride;
+    const short* ts = tap_src + (size_t)r0 * kTapStride;
+    for (int e = tid; e < R * kTapStride / EP; e += nth) cp_async<16>(sw + e * EP, tw + e * EP, true);
+    for (int e = tid; e < R * kTapStride / 4; e += nth) cp_async<8>(ssrc + e * 4, ts + e * 4, true);
   }
+  if (sdk)
+    for (int e = tid; e < D; e += nth) sseg[e] = L.seg[(m - L.m_lo) * D + e] - r0;
+  cp_async_wait_all();
+  const int am = abs(m), lmax = L.lmax;
   const int N = L.N;
   const T tp = (T)(2.0 * M_PI / prm.L);
   const int w = tid % W, rl = tid / W, nrl = nth / W;
@@ -193,14 +212,15 @@ __global__ void __launch_bounds__(256) k_local(RowLayout L, const c2<TIN>* __res
     for (int r = rl; r < R; r += nrl) {
       const C f0 = tile[r * W + w];
       T ax = noise * f0.x, ay = noise * f0.y;
+      Taps<T> tap;
+      tap.load(sw, ssrc, r);
 #pragma unroll
       for (int n2o = 0; n2o < 3; ++n2o) {
         T sx = 0, sy = 0;
 #pragma unroll
         for (int l1o = 0; l1o < 3; ++l1o) {
-          const int t = r * 9 + l1o * 3 + n2o;
-          const T wt = sw[t];
-          const C fs = tile[ssrc[t] * W + w];
+          const T wt = tap.w[l1o * 3 + n2o];
+          const C fs = tile[tap.src[l1o * 3 + n2o] * W + w];
           sx = fma(wt, fs.x, sx);
           sy = fma(wt, fs.y, sy);
         }
@@ -237,8 +257,8 @@ __global__ void __launch_bounds__(256) k_local(RowLayout L, const c2<TIN>* __res
 
 template <typename T> static size_t local_smem(const hp_plan* p, int W) {
   const int rmax = (p->lmax + 1) * (p->lmax + 1);
-  return local_tile_bytes<T>(rmax, W) + ((size_t)rmax * 9 * sizeof(T) + 15) / 16 * 16 +
-         sizeof(int) * ((p->D + 3) / 4 * 4) + sizeof(short) * (size_t)rmax * 9;
+  return local_tile_bytes<T>(rmax, W) + (sizeof(T) + sizeof(short)) * (size_t)rmax * kTapStride +
+         sizeof(int) * ((p->D + 3) / 4 * 4);
 }
 template <typename T> static const T* tap_table(const hp_plan* p);
 template <> const double* tap_table<double>(const hp_plan* p) { return p->tap_wr; }
@@ -735,10 +755,10 @@ static int local_w_launch(hp_plan* p, const c2<TIN>* F, c2<T>* G, const c2<T>* G
   ProfScope _ps(p, "deriv.local", s);
   if (p->ndim == 3) {
     HP_CUDA_TRY(cudaFuncSetAttribute(k_local<T, W, 3, TIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsm));
-    k_local<T, W, 3, TIN><<<grid, 256, lsm, s>>>(p->layout(), F, G, taps, Gx, so3d_table<T>(p), prm, cpb);
+    k_local<T, W, 3, TIN><<<grid, 256, lsm, s>>>(p->layout(), F, G, taps, p->tap_src, Gx, so3d_table<T>(p), prm, cpb);
   } else {
     HP_CUDA_TRY(cudaFuncSetAttribute(k_local<T, W, 2, TIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsm));
-    k_local<T, W, 2, TIN><<<grid, 256, lsm, s>>>(p->layout(), F, G, taps, Gx, so3d_table<T>(p), prm, cpb);
+    k_local<T, W, 2, TIN><<<grid, 256, lsm, s>>>(p->layout(), F, G, taps, p->tap_src, Gx, so3d_table<T>(p), prm, cpb);
   }
   HP_CUDA_TRY(cudaGetLastError());
   return HP_OK;
@@ -1056,30 +1076,25 @@ int hp_derivative_eval_prm(hp_plan* p, const DerivParams& prm, const double2* Fe
 // from which the gradients of the gravity scales and of G follow per point:
 // Re<lam, -D_i sum_q MR_i[q] ..> = d_i Im sum_q MR_i[q] t[q], and c_ij u.  One
 // read of F and lam replaces three passes of k_local with a dot each and the
-// noise dot (B = 12, 24^3: 0.99 -> 0.24 ms).
+// noise dot (B = 12, 24^3: 0.99 -> 0.21 ms).
 template <int W, int NDIM>
 __global__ void __launch_bounds__(256) k_local_dots(RowLayout L, const double2* __restrict__ F,
                                                     const double2* __restrict__ lam, const double* __restrict__ tap_wr,
-                                                    DerivParams prm, int cpb, int half, double scale,
+                                                    const short* __restrict__ tap_src, DerivParams prm, int cpb, int half, double scale,
                                                     double* __restrict__ acc, int nblocks, int slot) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int D = 2 * L.lmax + 1, rmax = (L.lmax + 1) * (L.lmax + 1);
   double2* tile = reinterpret_cast<double2*>(smraw);                                   // [R][W]
-  double* sw = reinterpret_cast<double*>(smraw + local_tile_bytes<double>(rmax, W));   // [R][9]
-  short* ssrc = reinterpret_cast<short*>(sw + (size_t)rmax * 9);                       // [R][9]
+  double* sw = reinterpret_cast<double*>(smraw + local_tile_bytes<double>(rmax, W));   // [R][kTapStride]
+  short* ssrc = reinterpret_cast<short*>(sw + (size_t)rmax * kTapStride);              // [R][kTapStride]
   const int m = (int)blockIdx.y + L.m_lo;
   const int r0 = L.seg[(m - L.m_lo) * D];
   const int r1 = (m + 1 <= L.lmax) ? L.seg[(m + 1 - L.m_lo) * D] : (int)L.nrows;
-  const int R = r1 - r0, am = abs(m), lmax = L.lmax, N = L.N;
+  const int R = r1 - r0, N = L.N;
   const int tid = threadIdx.x, nth = blockDim.x;
-  for (int e = tid; e < R * 9; e += nth) {
-    sw[e] = tap_wr[(size_t)r0 * 9 + e];
-    const char4 q = L.rows[r0 + e / 9];
-    const int t = e % 9, l1 = q.x + t / 3 - 1, n1 = q.z - (t % 3 - 1), an1 = abs(n1);
-    int src = 0;
-    if (l1 >= 0 && l1 <= lmax && am <= l1 && an1 <= l1)
-      src = L.seg[(m - L.m_lo) * D + n1 + lmax] - r0 + l1 - (am > an1 ? am : an1);
-    ssrc[e] = (short)src;
+  for (int e = tid; e < R * kTapStride; e += nth) {
+    sw[e] = tap_wr[(size_t)r0 * kTapStride + e];
+    ssrc[e] = tap_src[(size_t)r0 * kTapStride + e];
   }
   const double tp = 2.0 * M_PI / prm.L, weight = scale * (half && m > 0 ? 2.0 : 1.0);
   const int w = tid % W, rl = tid / W, nrl = nth / W;
@@ -1110,7 +1125,7 @@ __global__ void __launch_bounds__(256) k_local_dots(RowLayout L, const double2* 
         double sx = 0.0, sy = 0.0;
 #pragma unroll
         for (int l1o = 0; l1o < 3; ++l1o) {
-          const int k = r * 9 + l1o * 3 + q;
+          const int k = r * kTapStride + l1o * 3 + q;
           const double wt = sw[k];
           const double2 fs = tile[ssrc[k] * W + w];
           sx = fma(wt, fs.x, sx);
@@ -1173,7 +1188,7 @@ static int local_dots_launch(hp_plan* p, const double2* F, const double2* lam, d
   ProfScope _ps(p, "adj.dot", s);
   auto launch = [&](auto kern) -> int {
     HP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsm));
-    kern<<<grid, 256, lsm, s>>>(p->layout(), F, lam, p->tap_wr, prm, cpb, half, scale, acc, nblocks, slot);
+    kern<<<grid, 256, lsm, s>>>(p->layout(), F, lam, p->tap_wr, p->tap_src, prm, cpb, half, scale, acc, nblocks, slot);
     HP_CUDA_TRY(cudaGetLastError());
     return HP_OK;
   };

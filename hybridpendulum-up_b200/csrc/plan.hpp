@@ -20,6 +20,9 @@ struct RowLayout {
   const int* seg;                   // first row of segment (m, n): seg[(m-m_lo)*(2lmax+1) + n+lmax]
 };
 
+// taps per row in the tables: nine, padded to whole 16-byte reads
+constexpr int kTapStride = 12;
+
 struct hp_state;
 
 struct Buf {
@@ -59,8 +62,10 @@ struct hp_plan {
   // model
   bool has_model = false;
   hp_model model{};
-  double* tap_wr = nullptr;  // [row][9] real gravity tap weights, tap (l1-l+1)*3 + (n2+1)
+  // [row][kTapStride] real gravity tap weights, tap (l1-l+1)*3 + (n2+1), zeros behind
+  double* tap_wr = nullptr;
   float* tap_wr32 = nullptr;
+  short* tap_src = nullptr;  // [row][kTapStride] the tap's row, counted from the first row of its m group
   double2 mr1[3][3] = {};    // MR_i^1_{0 n2} of the model: [n2+1][i]
   double* den_mR = nullptr;  // [2][(2B)^3] density-side gravity multipliers (pendulum_reduced_den)
   // attitude diffusion sum_ij G1_ij F^l u_i^T u_j^T of the gyro-bias model:
@@ -152,7 +157,7 @@ void hp_tune_apply_cached(hp_plan* p);
 int hp_tables_build(hp_plan* p);
 int hp_twiddles_init();
 int hp_build_gravity_taps(hp_plan* p);
-// the weights of W Grav W^-1, W = diag(2l+1), in the plan's compute precision (out: [row][9])
+// the weights of W Grav W^-1, W = diag(2l+1), in the plan's compute precision (out: [row][kTapStride])
 int hp_adjoint_gravity_taps(hp_plan* p, void* out, cudaStream_t s);
 int hp_full_to_internal(hp_plan* p, const double2* Ffull, double2* Fint, cudaStream_t s);
 // the same of the projection onto the real-density subspace, (F + C F) / 2
@@ -239,6 +244,9 @@ int tc_beta_errors(hp_plan* p, int* count);
 }  // namespace hp
 int hp_forward_internal(hp_plan* p, const void* f, int complex_in, double2* Fint, cudaStream_t s);
 int hp_forward_internal64(hp_plan* p, const double* f, double2* Fint, cudaStream_t s);
+// FP64 SO(3) transforms of nb real functions without omega axes (HP_REAL plans): rows [row][nb]
+int hp_so3_forward64(hp_plan* p, const double* f, double2* rows, long long nb, cudaStream_t s);
+int hp_so3_backward64(hp_plan* p, const double2* rows, double* f, long long nb, cudaStream_t s);
 // inverse (scaled 1/nx) / forward omega FFT of every row, in the plan's compute precision
 int hp_omega_ifft_rows(hp_plan* p, const double2* in, void* out, cudaStream_t s);
 int hp_omega_fft_rows(hp_plan* p, void* inout, cudaStream_t s);
