@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(128) k_synth_beta(long long nx, const c2<T>* _
 
 template <int B, typename T, bool CPLX>
 __global__ void __launch_bounds__(Synth2Cfg<B, T, CPLX>::NT, Synth2Cfg<B, T, CPLX>::MINB)
-    k_synth_ga(const c2<T>* __restrict__ G, void* __restrict__ fout, long long w0) {
+    k_synth_ga(const c2<T>* __restrict__ G, void* __restrict__ fout, long long w0, long long nx) {
   using C = c2<T>;
   using Cfg = Synth2Cfg<B, T, CPLX>;
   constexpr int NB2 = 2 * B, NM = Cfg::NM, NCOL = Cfg::NCOL, PA = Cfg::PA, NB = Cfg::NB, NT = Cfg::NT;
@@ -202,7 +202,9 @@ __global__ void __launch_bounds__(Synth2Cfg<B, T, CPLX>::NT, Synth2Cfg<B, T, CPL
                     (nbv * NB2 * VAL) % 16 == 0 && (NB2 * NB2 * VAL) % 16 == 0;
   if (bulk) fence_proxy_async_smem();
   __syncthreads();
-  // f[a + 2B (b + 2B (c + 2B w))]
+  // f[a + 2B (b + 2B (c + 2B w))]; runs go [c][p], the points past the end of a
+  // batch that PA does not divide are left out
+  const int pc = (int)min((long long)PA, nx - w0 - wb * PA);
   auto dst = [&](int run) -> unsigned char* {
     const long long w = w0 + wb * PA + run % PA;
     return reinterpret_cast<unsigned char*>(fout) + (((size_t)w * NB2 + run / PA) * NB2 + b0) * NB2 * VAL;
@@ -211,11 +213,12 @@ __global__ void __launch_bounds__(Synth2Cfg<B, T, CPLX>::NT, Synth2Cfg<B, T, CPL
     const uint64_t pol = l2_policy_evict_first();
     if ((tid & 31) == 0)
       for (int run = tid >> 5; run < PA * NB2; run += NT / 32)
-        bulk_s2g(dst(run), smraw + (size_t)run * RS, (unsigned)(nbv * NB2 * VAL), pol);
+        if (run % PA < pc) bulk_s2g(dst(run), smraw + (size_t)run * RS, (unsigned)(nbv * NB2 * VAL), pol);
     bulk_commit();
     bulk_wait_all();   // shared memory must outlive the copies reading it
   } else {
     for (int run = tid >> 5; run < PA * NB2; run += NT / 32) {
+      if (run % PA >= pc) continue;
       T* o = reinterpret_cast<T*>(dst(run));
       const T* src = reinterpret_cast<const T*>(smraw + (size_t)run * RS);
       for (int e = tid & 31; e < nbv * NB2 * (VAL / (int)sizeof(T)); e += 32) o[e] = src[e];
@@ -235,9 +238,10 @@ __global__ void k_dsyn_table(RowLayout L, const T* __restrict__ wig, int DS, T* 
 }
 
 template <int B, typename T, bool CPLX>
-int synth2_launch(hp_plan* p, const c2<T>* Fp, void* f, cudaStream_t s) {
+int synth2_launch(hp_plan* p, const c2<T>* Fp, void* f, long long nx, cudaStream_t s) {
   using C = c2<T>;
   using Cfg = Synth2Cfg<B, T, CPLX>;
+  if (tw_init() != 0) { hp_set_error("twiddle table upload failed"); return HP_ERR_CUDA; }
   constexpr int NB2 = 2 * B, NM = Cfg::NM, PA = Cfg::PA, NB = Cfg::NB, NPAIR = NM * (2 * B - 1), DS = (NB2 + 3) / 4 * 4;
   int st = HP_OK;
   const char* key = CPLX ? "tf.pairs_c" : "tf.pairs_r";
@@ -262,24 +266,24 @@ int synth2_launch(hp_plan* p, const c2<T>* Fp, void* f, cudaStream_t s) {
   }
   const long long per_w = (long long)NM * NB2 * NB2 * (long long)sizeof(C);
   long long nwc = std::max(32LL, kSynthG / per_w / 32 * 32);
-  nwc = std::min(nwc, (p->nx + 31) / 32 * 32);
+  nwc = std::min(nwc, (nx + 31) / 32 * 32);
   C* G = (C*)p->ws_get("tf.G", (size_t)per_w * nwc, &st);
   if (st) return st;
   constexpr size_t smem = (size_t)Cfg::bytes(NB, PA);
   HP_CUDA_TRY(cudaFuncSetAttribute(k_synth_ga<B, T, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   constexpr int NGRP = (NB2 + NB - 1) / NB;
-  for (long long w0 = 0; w0 < p->nx; w0 += nwc) {
-    const long long nw = std::min(nwc, p->nx - w0);   // a multiple of 4 (N is even), so of PA
+  for (long long w0 = 0; w0 < nx; w0 += nwc) {
+    const long long nw = std::min(nwc, nx - w0);
     {
       ProfScope _ps(p, "tf.synth.beta", s);
       constexpr size_t dsm = 4 * sizeof(T) * (size_t)((B + 3) / 4 * 4 * DS);
       HP_CUDA_TRY(cudaFuncSetAttribute(k_synth_beta<B, T, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm));
       k_synth_beta<B, T, CPLX><<<dim3((unsigned)((nw + 31) / 32), (unsigned)((NPAIR + 3) / 4)), 128, dsm, s>>>(
-          p->nx, Fp, dtab, dpairs, NPAIR, G, w0, nw);
+          nx, Fp, dtab, dpairs, NPAIR, G, w0, nw);
       HP_CUDA_TRY(cudaGetLastError());
     }
     ProfScope _ps(p, "tf.synth", s);
-    k_synth_ga<B, T, CPLX><<<(unsigned)(nw / PA * NGRP), Cfg::NT, smem, s>>>(G, f, w0);
+    k_synth_ga<B, T, CPLX><<<(unsigned)((nw + PA - 1) / PA * NGRP), Cfg::NT, smem, s>>>(G, f, w0, nx);
     HP_CUDA_TRY(cudaGetLastError());
   }
   return HP_OK;

@@ -234,10 +234,11 @@ static int omega_fft_any(hp_plan* p, const c2<Tin>* in, c2<T>* out, bool inv, cu
   extern template int synth_launch<b, float, true>(hp_plan*, const float2*, void*, cudaStream_t);         \
   extern template int synth_launch<b, double, false>(hp_plan*, const double2*, void*, cudaStream_t);      \
   extern template int synth_launch<b, double, true>(hp_plan*, const double2*, void*, cudaStream_t);       \
-  extern template int anal2_launch<b, float, false>(hp_plan*, const void*, const double*, float2*, cudaStream_t);  \
-  extern template int anal2_launch<b, float, true>(hp_plan*, const void*, const double*, float2*, cudaStream_t);   \
-  extern template int anal2_launch<b, double, false>(hp_plan*, const void*, const double*, double2*, cudaStream_t); \
-  extern template int anal2_launch<b, double, true>(hp_plan*, const void*, const double*, double2*, cudaStream_t);
+  extern template int anal2_launch<b, float, false>(hp_plan*, const void*, const double*, float2*, long long, cudaStream_t);  \
+  extern template int anal2_launch<b, float, true>(hp_plan*, const void*, const double*, float2*, long long, cudaStream_t);   \
+  extern template int anal2_launch<b, double, false>(hp_plan*, const void*, const double*, double2*, long long, cudaStream_t); \
+  extern template int anal2_launch<b, double, true>(hp_plan*, const void*, const double*, double2*, long long, cudaStream_t); \
+  extern template int synth2_launch<b, double, false>(hp_plan*, const double2*, void*, long long, cudaStream_t);
 HP_FOR_EACH_B(X)
 #undef X
 
@@ -292,7 +293,7 @@ static int backward_T(hp_plan* p, const double2* Fint, void* f, int complex_out,
 template <typename T, bool CPLX>
 static int anal2_any(hp_plan* p, const void* f, const double* mult, c2<T>* out, cudaStream_t s) {
   switch (p->B) {
-#define X(b) case b: return anal2_launch<b, T, CPLX>(p, f, mult, out, s);
+#define X(b) case b: return anal2_launch<b, T, CPLX>(p, f, mult, out, p->nx, s);
     HP_FOR_EACH_B(X)
 #undef X
     default:
@@ -307,11 +308,8 @@ static int forward_rows_T(hp_plan* p, const void* f, int complex_in, const doubl
   using C = c2<T>;
   int st = HP_OK;
   const size_t fb = sizeof(C) * (size_t)p->nrows * p->nx;
-  C* t1 = (C*)p->ws_get("tf.t1", fb, &st);
-  if (st) return st;
   C* t2 = (C*)p->ws_get("tf.t2", fb, &st);
   if (st) return st;
-  (void)t1;
   st = complex_in ? anal2_any<T, true>(p, f, mult, t2, s) : anal2_any<T, false>(p, f, mult, t2, s);
   if (st) return st;
   return omega_fft_any<T, T>(p, t2, out, false, s);
@@ -320,17 +318,21 @@ static int forward_rows_T(hp_plan* p, const void* f, int complex_in, const doubl
 template <typename T>
 static int forward_T(hp_plan* p, const void* f, int complex_in, double2* Fint, cudaStream_t s) {
   using C = c2<T>;
-  int st = HP_OK;
-  C* t3 = (C*)p->ws_get("tf.t1", sizeof(C) * (size_t)p->nrows * p->nx, &st);  // free again after the transpose
-  if (st) return st;
-  st = forward_rows_T<T>(p, f, complex_in, nullptr, t3, s);
-  if (st) return st;
-  // to FP64 rows
-  const long long n = p->nrows * p->nx;
-  ProfScope _ps(p, "convert", s);
-  k_to_c64<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(t3, Fint, n);
-  HP_CUDA_TRY(cudaGetLastError());
-  return HP_OK;
+  if constexpr (sizeof(T) == 8) {   // the rows are FP64 already
+    return forward_rows_T<T>(p, f, complex_in, nullptr, Fint, s);
+  } else {
+    int st = HP_OK;
+    C* t3 = (C*)p->ws_get("tf.t1", sizeof(C) * (size_t)p->nrows * p->nx, &st);
+    if (st) return st;
+    st = forward_rows_T<T>(p, f, complex_in, nullptr, t3, s);
+    if (st) return st;
+    // to FP64 rows
+    const long long n = p->nrows * p->nx;
+    ProfScope _ps(p, "convert", s);
+    k_to_c64<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(t3, Fint, n);
+    HP_CUDA_TRY(cudaGetLastError());
+    return HP_OK;
+  }
 }
 
 int hp_backward_internal(hp_plan* p, const double2* Fint, void* f, int complex_out, cudaStream_t s) {
@@ -356,6 +358,29 @@ int hp_forward_internal_T(hp_plan* p, const void* f, const double* mult, void* o
   const int cplx = p->symmetry == HP_COMPLEX;
   if (p->precision == HP_FP64) return forward_rows_T<double>(p, f, cplx, mult, (double2*)out, s);
   return forward_rows_T<float>(p, f, cplx, mult, (float2*)out, s);
+}
+
+// FP64 SO(3) transforms of nb real functions f (2B, 2B, 2B, nb) without omega
+// axes, HP_REAL plans of any precision: rows [row][nb].
+int hp_so3_forward64(hp_plan* p, const double* f, double2* rows, long long nb, cudaStream_t s) {
+  switch (p->B) {
+#define X(b) case b: return anal2_launch<b, double, false>(p, f, nullptr, rows, nb, s);
+    HP_FOR_EACH_B(X)
+#undef X
+    default:
+      hp_set_error("bandlimit B not supported (2..32)");
+      return HP_ERR_UNSUPPORTED;
+  }
+}
+int hp_so3_backward64(hp_plan* p, const double2* rows, double* f, long long nb, cudaStream_t s) {
+  switch (p->B) {
+#define X(b) case b: return synth2_launch<b, double, false>(p, rows, f, nb, s);
+    HP_FOR_EACH_B(X)
+#undef X
+    default:
+      hp_set_error("bandlimit B not supported (2..32)");
+      return HP_ERR_UNSUPPORTED;
+  }
 }
 
 // Forward transform in FP64 whatever the plan's precision (initial densities).

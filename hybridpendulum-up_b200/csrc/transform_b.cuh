@@ -106,135 +106,166 @@ template <int B, typename T, bool CPLX>
 int synth_launch(hp_plan* p, const c2<T>* Fp, void* f, cudaStream_t s) {
   if (tw_init() != 0) { hp_set_error("twiddle table upload failed"); return HP_ERR_CUDA; }
   if constexpr (!CPLX && RealSynthCfg<B, T>::ok) return synth_real_launch<B, T>(p, Fp, reinterpret_cast<T*>(f), s);
-  else return synth2_launch<B, T, CPLX>(p, Fp, f, s);
+  else return synth2_launch<B, T, CPLX>(p, Fp, f, p->nx, s);
 }
 
 // ----------------------------------------- analysis without atomics ----
 // Stage 1 (k_anal_ag): block = (beta, chunk of PA omega points).  For each
 // omega point the alpha FFT over a and the gamma FFT over c of f(., b, ., w)
 // (times an optional grid multiplier) give Q_b[m][n]; it is written to
-// Qg[(m, n bin)][b][w] with the chunk's omega points consecutive.
+// Qg[(m, n bin)][b][w] with the chunk's omega points consecutive.  Bound by the
+// shared-memory pipe: unpadded tiles put the lanes of a warp on one to four
+// banks in the reads of both FFTs and of the store, with one or two blocks of
+// 256 threads per SM.  16 x 16 omega points, before / now (us): B = 16 FP32 125 /
+// 38, FP64 240 / 67; B = 32 FP32 792 / 304, FP64 1778 / 891; 16^3, B = 10 FP64 318
+// / 109.
+// nx: the number of omega points (the plan's, or a batch of functions on SO(3)).
 // Stage 2 (k_anal_beta): thread = ((m, n) pair, omega point), all l of the
 // pair: F^l_mn[w] = sum_b w_b d^l_mn(beta_b) Q_b[m][n][w], written straight
 // into the [row][omega] layout.  Every output has one owner: no atomics.
-template <int B, typename T, int PA, bool CPLX>
-__global__ void __launch_bounds__(B >= 24 ? 128 : 256, B >= 24 && sizeof(T) == 4 ? 3 : 1)
-    k_anal_ag(const void* __restrict__ fin, const double* __restrict__ mult,
-                                                 c2<T>* __restrict__ Qg, long long w0, long long nwc) {
+// Shapes of stage 1.  Rows in shared memory are padded so that lanes on
+// consecutive rows hit distinct banks: input lines (2B values of one (omega,
+// gamma) column) start an odd number of 16-byte units apart and are read 16
+// bytes at a time; rows of the output tile [omega][m][2B] are 2B + 1 values, an
+// omega point's rows an odd number of values apart.
+template <int B, typename T, bool CPLX> struct AnalCfg {
   using C = c2<T>;
-  constexpr int NB2 = 2 * B, lmax = B - 1, D = 2 * lmax + 1;
-  constexpr int NM = CPLX ? D : B;
-  constexpr int MLO = CPLX ? -lmax : 0;
+  static constexpr int NB2 = 2 * B, NM = CPLX ? 2 * B - 1 : B;
+  static constexpr int items = CPLX ? 2 * B : B;    // alpha items per omega point
+  static constexpr int NT = 128;
+  static constexpr int VAL = (int)sizeof(T) * (CPLX ? 2 : 1);       // bytes of a density value
+  static constexpr int LS = ((NB2 * VAL + 15) / 16) | 1;            // 16-byte units per input line
+  static constexpr int GQ = NB2 + 1, TSQ = (NM * GQ) | 1;           // output row, output omega point (values)
+  static constexpr long long bytes(int pa) {
+    const long long in = (long long)pa * NB2 * LS * 16, q = (long long)pa * TSQ * (long long)sizeof(C);
+    const long long tile = ((in > q ? in : q) + 15) / 16 * 16;
+    return tile + (CPLX ? 0 : (long long)NB2 * LS * 16);            // + this beta's grid multiplier (real densities)
+  }
+  // the largest omega batch with one alpha item per thread and three blocks per
+  // SM; at least 4 (32-byte stores in FP32) where two blocks allow it
+  static constexpr int pick() {
+    int pa = 16;
+    while (pa > 1 && (pa * items > NT || bytes(pa) > (pa > 4 ? 72 : 110) * 1024)) pa /= 2;
+    return pa;
+  }
+  static constexpr int PA = pick();
+  // blocks per SM that the registers are held to
+  static constexpr int MINB = sizeof(T) == 4 ? (NB2 <= 24 ? 6 : NB2 <= 32 ? 4 : NB2 <= 48 ? 3 : 2)
+                                             : (NB2 <= 12 ? 6 : NB2 <= 20 ? 4 : NB2 <= 32 ? 3 : 2);
+};
+
+// 16-byte reads of N consecutive values (16-byte aligned)
+template <int N> __device__ __forceinline__ void load_line(const float* s, float (&v)[N]) {
+#pragma unroll
+  for (int i = 0; i + 4 <= N; i += 4) {
+    const float4 q = *reinterpret_cast<const float4*>(s + i);
+    v[i] = q.x; v[i + 1] = q.y; v[i + 2] = q.z; v[i + 3] = q.w;
+  }
+  if constexpr (N % 4) {
+    const float2 q = *reinterpret_cast<const float2*>(s + N - 2);
+    v[N - 2] = q.x; v[N - 1] = q.y;
+  }
+}
+template <int N> __device__ __forceinline__ void load_line(const double* s, double (&v)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; i += 2) {
+    const double2 q = *reinterpret_cast<const double2*>(s + i);
+    v[i] = q.x; v[i + 1] = q.y;
+  }
+}
+
+template <int B, typename T, int PA, bool CPLX>
+__global__ void __launch_bounds__(AnalCfg<B, T, CPLX>::NT, (AnalCfg<B, T, CPLX>::MINB))
+    k_anal_ag(const void* __restrict__ fin, const double* __restrict__ mult, c2<T>* __restrict__ Qg, long long w0,
+              long long nwc) {
+  using C = c2<T>;
+  using Cfg = AnalCfg<B, T, CPLX>;
+  constexpr int NB2 = 2 * B, NM = Cfg::NM, MLO = CPLX ? -(B - 1) : 0;
+  constexpr int NT = Cfg::NT, VAL = Cfg::VAL, LB = Cfg::LS * 16, GQ = Cfg::GQ, TSQ = Cfg::TSQ;
   extern __shared__ __align__(16) unsigned char smraw[];
-  // input tile [PA][c][a] (complex, or real values for real densities); the
-  // alpha stage reads its lines into registers before a barrier, so its
-  // output [PA][m][c or q] reuses the same shared memory
-  C* sIn = reinterpret_cast<C*>(smraw);
-  T* sInR = reinterpret_cast<T*>(smraw);
+  // input lines [PA][c] of LB bytes; the alpha stage reads its lines into
+  // registers before a barrier, so its output [PA][m][c or q] reuses the space
   C* sQ = reinterpret_cast<C*>(smraw);
+  unsigned char* smult = smraw + Cfg::bytes(PA) - (CPLX ? 0 : (size_t)NB2 * LB);   // [c] lines of the multiplier
   const int b = blockIdx.y;
   const long long wl0 = (long long)blockIdx.x * PA;                       // chunk-local omega
   const int pc = (int)min((long long)PA, nwc - wl0);
-  const int tid = threadIdx.x, nth = blockDim.x;
-  const int NG = NB2 * NB2;
-  constexpr long long TILE = (long long)PA * (2LL * NM * NB2 > (long long)NB2 * NB2 * (CPLX ? 2 : 1)
-                                               ? 2LL * NM * NB2 : (long long)NB2 * NB2 * (CPLX ? 2 : 1));
-  T* smult = reinterpret_cast<T*>(smraw) + TILE;   // [c][a] multiplier of this beta (real densities)
-  // Real densities whose 2B-runs are 16-byte aligned: every run of 2B
-  // consecutive a arrives by 16-byte asynchronous copies (all in flight at
-  // once), the grid multiplier slice of this beta is staged beside it and
-  // applied when the alpha stage reads its lines.
-  constexpr bool ASYNC = !CPLX && (NB2 * sizeof(T)) % 16 == 0;
-  const bool async_ok = ASYNC && (reinterpret_cast<unsigned long long>(fin) & 15ull) == 0;
-  if (async_ok) {
-    constexpr int VPR = NB2 * (int)sizeof(T) / 16;                       // 16-byte pieces per run
-    for (int e = tid; e < pc * NB2 * VPR; e += nth) {
-      const int run = e / VPR, piece = e % VPR, pp = run / NB2, cc = run % NB2;
-      const long long w = w0 + wl0 + pp;
-      const long long gi = (long long)NB2 * ((long long)b + NB2 * ((long long)cc + NB2 * w));
-      cp_async<16>(sInR + (size_t)run * NB2 + piece * (16 / sizeof(T)),
-                   reinterpret_cast<const T*>(fin) + gi + piece * (16 / sizeof(T)), true);
+  const int tid = threadIdx.x;
+  // load f(., b, c, w): 2B consecutive a per (c, w), by asynchronous copies, all
+  // in flight at once (pieces of 16 bytes, 8 where 2B values are not a multiple
+  // of 16 bytes); a density buffer off a 16-byte boundary is copied by values
+  constexpr int PB = (NB2 * VAL) % 16 == 0 ? 16 : 8, PPR = NB2 * VAL / PB;
+  const unsigned char* src = reinterpret_cast<const unsigned char*>(fin) + ((w0 + wl0) * NB2 * NB2 + b) * (size_t)(NB2 * VAL);
+  if ((reinterpret_cast<unsigned long long>(fin) & 15ull) == 0) {
+    for (int e = tid; e < pc * NB2 * PPR; e += NT) {
+      const int run = e / PPR, piece = e - run * PPR;
+      cp_async<PB>(smraw + (size_t)run * LB + piece * PB, src + (size_t)run * (NB2 * NB2 * VAL) + piece * PB, true);
     }
-    for (int e = tid; e < NG; e += nth) {
-      const int cc = e / NB2, a = e % NB2;
-      smult[e] = mult ? (T)mult[a + NB2 * (b + NB2 * cc)] : (T)1;
-    }
-    cp_async_wait_all();
-  } else
-  // load f(a, b, c, w) for this beta: runs of 2B consecutive a
-  for (int e = tid; e < pc * NG; e += nth) {
-    const int pp = e / NG, r = e % NG, cc = r / NB2, a = r % NB2;
-    const long long w = w0 + wl0 + pp;
-    const long long gi = (long long)a + NB2 * ((long long)b + NB2 * ((long long)cc + NB2 * w));
-    const T mv = mult ? (T)mult[a + NB2 * (b + NB2 * cc)] : (T)1;
-    if (CPLX) {
-      C v = reinterpret_cast<const C*>(fin)[gi];
-      v.x *= mv;
-      v.y *= mv;
-      sIn[e] = v;
-    } else {
-      sInR[e] = reinterpret_cast<const T*>(fin)[gi] * mv;
+  } else {
+    for (int e = tid; e < pc * NB2 * (NB2 * VAL / (int)sizeof(T)); e += NT) {
+      constexpr int TPR = NB2 * VAL / (int)sizeof(T);
+      const int run = e / TPR, i = e - run * TPR;
+      reinterpret_cast<T*>(smraw + (size_t)run * LB)[i] = reinterpret_cast<const T*>(src + (size_t)run * (NB2 * NB2 * VAL))[i];
     }
   }
+  if (!CPLX && mult)   // the grid multiplier of this beta (density-gravity terms)
+    for (int e = tid; e < NB2 * NB2; e += NT) {
+      const int c = e / NB2, a = e % NB2;
+      reinterpret_cast<T*>(smult + (size_t)c * LB)[a] = (T)mult[a + NB2 * (b + NB2 * c)];
+    }
+  cp_async_wait_all();
   __syncthreads();
-  // alpha, one item per thread (the host keeps the item count within the
-  // block).  Real densities: item (p, c pair), columns c, c+1 share one complex
-  // FFT, z = f_c + i f_{c+1}: X_c[m] = (Z[m] + conj Z[-m]) / 2,
-  // X_{c+1}[m] = (Z[m] - conj Z[-m]) / 2i.  Complex densities: item (p, c).
+  // alpha, one item per thread.  Real densities: item (p, c), columns c and c + B
+  // share one complex FFT, z = f_c + i f_{c+B}: X_c[m] = (Z[m] + conj Z[-m]) / 2,
+  // X_{c+B}[m] = (Z[m] - conj Z[-m]) / 2i.  Complex densities: item (p, c).
   {
-    const int nitems = CPLX ? pc * NB2 : pc * B;
-    const bool act = tid < nitems;
-    const int pp = CPLX ? tid / NB2 : tid / B;
-    const int c0 = CPLX ? tid % NB2 : 2 * (tid % B);
+    const bool act = tid < pc * Cfg::items;
+    const int pp = tid / Cfg::items, c = tid % Cfg::items;
     C x[NB2];
     if (act) {
-      if (CPLX) {
-        const C* src = sIn + (size_t)tid * NB2;
+      const unsigned char* line = smraw + (size_t)(pp * NB2 + c) * LB;
+      if constexpr (CPLX) {
+        const C* r = reinterpret_cast<const C*>(line);
 #pragma unroll
-        for (int a = 0; a < NB2; ++a) x[a] = src[a];
-      } else if (async_ok) {
-        const T* r0 = sInR + ((size_t)pp * NB2 + c0) * NB2;
-        const T* r1 = r0 + NB2;
-        const T* m0 = smult + (size_t)c0 * NB2;
-        const T* m1 = m0 + NB2;
-#pragma unroll
-        for (int a = 0; a < NB2; ++a) { x[a].x = r0[a] * m0[a]; x[a].y = r1[a] * m1[a]; }
+        for (int a = 0; a < NB2; ++a) x[a] = r[a];
       } else {
-        const T* r0 = sInR + ((size_t)pp * NB2 + c0) * NB2;
-        const T* r1 = r0 + NB2;
+        T u[NB2], v[NB2];
+        load_line<NB2>(reinterpret_cast<const T*>(line), u);
+        load_line<NB2>(reinterpret_cast<const T*>(line + (size_t)B * LB), v);
 #pragma unroll
-        for (int a = 0; a < NB2; ++a) { x[a].x = r0[a]; x[a].y = r1[a]; }
+        for (int a = 0; a < NB2; ++a) x[a] = mk(u[a], v[a]);
+        if (mult) {
+          load_line<NB2>(reinterpret_cast<const T*>(smult + (size_t)c * LB), u);
+          load_line<NB2>(reinterpret_cast<const T*>(smult + (size_t)(c + B) * LB), v);
+#pragma unroll
+          for (int a = 0; a < NB2; ++a) { x[a].x *= u[a]; x[a].y *= v[a]; }
+        }
       }
     }
     __syncthreads();
     if (act) {
       fft<NB2, true>(x);
-      C* dst = sQ + (size_t)pp * NM * NB2 + c0;
-      if (CPLX) {
+      C* dst = sQ + (size_t)pp * TSQ + c;
+      if constexpr (CPLX) {
 #pragma unroll
         for (int mi = 0; mi < NM; ++mi) {
           const int m = mi + MLO;
-          dst[(size_t)mi * NB2] = x[m >= 0 ? m : m + NB2];
+          dst[mi * GQ] = x[m >= 0 ? m : m + NB2];
         }
       } else {
 #pragma unroll
         for (int m = 0; m < NM; ++m) {
           const C zp = x[m], zm = x[(NB2 - m) % NB2];
-          C u, v;
-          u.x = (T)0.5 * (zp.x + zm.x);
-          u.y = (T)0.5 * (zp.y - zm.y);
-          v.x = (T)0.5 * (zp.y + zm.y);
-          v.y = (T)0.5 * (zm.x - zp.x);
-          dst[(size_t)m * NB2] = u;
-          dst[(size_t)m * NB2 + 1] = v;
+          dst[m * GQ] = mk((T)0.5 * (zp.x + zm.x), (T)0.5 * (zp.y - zm.y));
+          dst[m * GQ + B] = mk((T)0.5 * (zp.y + zm.y), (T)0.5 * (zm.x - zp.x));
         }
       }
     }
   }
   __syncthreads();
   // gamma: item (p, m): FFT(+) over c, in place (bins n mod 2B)
-  for (int it = tid; it < pc * NM; it += nth) {
-    C* row = sQ + (size_t)it * NB2;
+  for (int it = tid; it < pc * NM; it += NT) {
+    C* row = sQ + (size_t)(it / NM) * TSQ + (it % NM) * GQ;
     C x[NB2];
 #pragma unroll
     for (int j = 0; j < NB2; ++j) x[j] = row[j];
@@ -244,9 +275,18 @@ __global__ void __launch_bounds__(B >= 24 ? 128 : 256, B >= 24 && sizeof(T) == 4
   }
   __syncthreads();
   // store: Qg[((m * 2B + q) * 2B + b) * nwc + w], consecutive omega points
-  for (int e = tid; e < NM * NB2 * pc; e += nth) {
-    const int pp = e % pc, mq = e / pc;
-    Qg[((long long)mq * NB2 + b) * nwc + wl0 + pp] = sQ[(size_t)pp * NM * NB2 + mq];
+  C* out = Qg + (long long)b * nwc + wl0;
+  if (pc == PA) {
+#pragma unroll 4
+    for (int e = tid; e < NM * NB2 * PA; e += NT) {
+      const int pp = e % PA, mq = e / PA;
+      out[(long long)mq * NB2 * nwc + pp] = sQ[pp * TSQ + mq + mq / NB2];
+    }
+  } else {
+    for (int e = tid; e < NM * NB2 * pc; e += NT) {
+      const int pp = e % pc, mq = e / pc;
+      out[(long long)mq * NB2 * nwc + pp] = sQ[pp * TSQ + mq + mq / NB2];
+    }
   }
 }
 
@@ -315,32 +355,8 @@ __global__ void k_dw_table(RowLayout L, const T* __restrict__ wig, const double*
   dw[t] = (T)(qw[b] * (double)wig[(size_t)b * L.nrows + r]);
 }
 
-// largest omega batch (16, 8, 4, 2, 1) whose stage-1 tiles fit the budget
-template <int B, typename T, bool CPLX> struct AnalCfg {
-  static constexpr int NM = CPLX ? 2 * B - 1 : B;
-  static constexpr long long in_w = (long long)(2 * B) * (2 * B) * (CPLX ? 2 : 1);   // T elements per omega
-  static constexpr long long q_w = 2LL * NM * (2 * B);
-  // tiles for pa omega points, plus (real densities) this beta's grid multiplier slice
-  static constexpr long long bytes(int pa) {
-    return (long long)pa * (in_w > q_w ? in_w : q_w) * (long long)sizeof(T) +
-           (CPLX ? 0 : (long long)(2 * B) * (2 * B) * (long long)sizeof(T));
-  }
-  static constexpr int items = CPLX ? 2 * B : B;    // alpha items per omega point
-  // threads per block: from B = 24 the 2B-point register FFTs need ~170-255
-  // registers, so two 128-thread blocks per SM overlap loads and FFTs
-  static constexpr int NT = B >= 24 ? 128 : 256;
-  // two resident blocks where a batch of 4 fits 110 KB, else one block of up to 220 KB
-  static constexpr long long cap() { return bytes(4) <= 110 * 1024 ? 110 * 1024 : 220 * 1024; }
-  static constexpr int pick() {
-    int pa = 16;
-    while (pa > 1 && (bytes(pa) > cap() || pa * items > NT)) pa /= 2;
-    return pa;
-  }
-  static constexpr int PA = pick();
-};
-
 template <int B, typename T, bool CPLX>
-int anal2_launch(hp_plan* p, const void* f, const double* mult, c2<T>* out, cudaStream_t s) {
+int anal2_launch(hp_plan* p, const void* f, const double* mult, c2<T>* out, long long nx, cudaStream_t s) {
   if (tw_init() != 0) { hp_set_error("twiddle table upload failed"); return HP_ERR_CUDA; }
   using C = c2<T>;
   using Cfg = AnalCfg<B, T, CPLX>;
@@ -373,12 +389,14 @@ int anal2_launch(hp_plan* p, const void* f, const double* mult, c2<T>* out, cuda
   // omega chunks keep the staged tiles within 2 GB
   const long long per_w = (long long)NM * NB2 * NB2 * (long long)sizeof(C);
   long long nwc = std::max(32LL, (2LL << 30) / per_w / 32 * 32);
-  nwc = std::min(nwc, (p->nx + 31) / 32 * 32);
+  nwc = std::min(nwc, (nx + 31) / 32 * 32);
+  RowLayout L = p->layout();
+  L.nx = nx;
   C* Qg = (C*)p->ws_get("tf.Q", (size_t)per_w * nwc, &st);
   if (st) return st;
   HP_CUDA_TRY(cudaFuncSetAttribute(k_anal_ag<B, T, PA, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  for (long long w0 = 0; w0 < p->nx; w0 += nwc) {
-    const long long nw = std::min(nwc, p->nx - w0);
+  for (long long w0 = 0; w0 < nx; w0 += nwc) {
+    const long long nw = std::min(nwc, nx - w0);
     {
       ProfScope _ps(p, "tf.anal.ag", s);
       dim3 ga((unsigned)((nw + PA - 1) / PA), (unsigned)NB2);
@@ -399,7 +417,7 @@ int anal2_launch(hp_plan* p, const void* f, const double* mult, c2<T>* out, cuda
     }
     ProfScope _ps(p, "tf.anal.beta", s);
     dim3 gb((unsigned)((nw + 31) / 32), (unsigned)((NPAIR + 7) / 8));
-    k_anal_beta<B, T, CPLX><<<gb, 256, 0, s>>>(p->layout(), Qg, dw, dpairs, NPAIR, out, w0, nw);
+    k_anal_beta<B, T, CPLX><<<gb, 256, 0, s>>>(L, Qg, dw, dpairs, NPAIR, out, w0, nw);
     HP_CUDA_TRY(cudaGetLastError());
   }
   return HP_OK;
@@ -414,8 +432,9 @@ int anal2_launch(hp_plan* p, const void* f, const double* mult, c2<T>* out, cuda
   template int synth_launch<b, float, true>(hp_plan*, const float2*, void*, cudaStream_t);         \
   template int synth_launch<b, double, false>(hp_plan*, const double2*, void*, cudaStream_t);      \
   template int synth_launch<b, double, true>(hp_plan*, const double2*, void*, cudaStream_t);       \
-  template int anal2_launch<b, float, false>(hp_plan*, const void*, const double*, float2*, cudaStream_t);  \
-  template int anal2_launch<b, float, true>(hp_plan*, const void*, const double*, float2*, cudaStream_t);   \
-  template int anal2_launch<b, double, false>(hp_plan*, const void*, const double*, double2*, cudaStream_t); \
-  template int anal2_launch<b, double, true>(hp_plan*, const void*, const double*, double2*, cudaStream_t);
+  template int anal2_launch<b, float, false>(hp_plan*, const void*, const double*, float2*, long long, cudaStream_t);  \
+  template int anal2_launch<b, float, true>(hp_plan*, const void*, const double*, float2*, long long, cudaStream_t);   \
+  template int anal2_launch<b, double, false>(hp_plan*, const void*, const double*, double2*, long long, cudaStream_t); \
+  template int anal2_launch<b, double, true>(hp_plan*, const void*, const double*, double2*, long long, cudaStream_t); \
+  template int synth2_launch<b, double, false>(hp_plan*, const double2*, void*, long long, cudaStream_t);
 #endif
