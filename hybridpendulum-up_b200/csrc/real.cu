@@ -18,6 +18,14 @@
 // with (t1, t2) = (sin, cos) for m, n of the same sign class, (cos, sin) otherwise
 // (ifftSO3.m:69-83).  Both 2-D sums over (alpha, gamma) are done separably per
 // (beta, function) block in shared memory; everything is FP64.
+//
+// HP_REAL plans take another route to the same numbers: the real coefficients
+// are F_r^l = T^l F_c^l (T^l)^H with F_c the complex ones and T^l the unitary of
+// fftSO3_prod.m:103-120 (two entries per row), so the transforms run on the
+// FFT kernels of the omega-batched transforms, the functions in the place of
+// omega points, and one pass changes the basis.  B = 16, 64 functions, forward
+// and backward: the direct sums 0.54 ms, this route 0.10 ms.  Complex plans hold
+// no tables for real functions and keep the direct sums.
 #include <cmath>
 #include <vector>
 #include "common.cuh"
@@ -195,6 +203,9 @@ __global__ void k_real_bwd_slice(int B, const double2* __restrict__ SF, double* 
   }
 }
 
+static int real_forward_rows(hp_plan* p, const double* f, double* F, int nb, cudaStream_t s);
+static int real_backward_rows(hp_plan* p, const double* F, double* f, int nb, cudaStream_t s);
+
 static const double* real_psi(hp_plan* p, int* st) {
   bool fresh = true;
   for (auto& kv : p->ws) if (kv.first == "real.psi") fresh = false;
@@ -220,10 +231,6 @@ extern "C" int hp_fftSO3_real_forward(hp_plan* p, const double* f, double* F, in
   const int B = p->B, N = 2 * B, D = p->D;
   const size_t nf = (size_t)N * N * N * nbatch, nF = (size_t)D * D * B * nbatch;
   int st = HP_OK;
-  const double* psi = real_psi(p, &st);
-  if (st) return st;
-  double2* S = (double2*)p->ws_get("real.S", sizeof(double2) * (size_t)D * D * N * nbatch, &st);
-  if (st) return st;
   const double* fd = f;
   double* Fd = F;
   if (mem == HP_HOST) {
@@ -234,7 +241,13 @@ extern "C" int hp_fftSO3_real_forward(hp_plan* p, const double* f, double* F, in
     HP_CUDA_TRY(cudaMemcpyAsync(a, f, sizeof(double) * nf, cudaMemcpyHostToDevice, p->stream));
     fd = a;
   }
-  {
+  if (p->symmetry == HP_REAL) {
+    HP_CHECK(real_forward_rows(p, fd, Fd, nbatch, p->stream));
+  } else {
+    const double* psi = real_psi(p, &st);
+    if (st) return st;
+    double2* S = (double2*)p->ws_get("real.S", sizeof(double2) * (size_t)D * D * N * nbatch, &st);
+    if (st) return st;
     ProfScope _ps(p, "real.fwd", p->stream);
     const size_t sm = sizeof(double) * N * N + sizeof(double2) * ((size_t)N * D + N);
     HP_CUDA_TRY(cudaFuncSetAttribute(k_real_fwd_slice, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -253,10 +266,6 @@ extern "C" int hp_fftSO3_real_backward(hp_plan* p, const double* F, double* f, i
   const int B = p->B, N = 2 * B, D = p->D;
   const size_t nf = (size_t)N * N * N * nbatch, nF = (size_t)D * D * B * nbatch;
   int st = HP_OK;
-  const double* psi = real_psi(p, &st);
-  if (st) return st;
-  double2* SF = (double2*)p->ws_get("real.S", sizeof(double2) * (size_t)D * D * N * nbatch, &st);
-  if (st) return st;
   const double* Fd = F;
   double* fd = f;
   if (mem == HP_HOST) {
@@ -267,7 +276,13 @@ extern "C" int hp_fftSO3_real_backward(hp_plan* p, const double* F, double* f, i
     HP_CUDA_TRY(cudaMemcpyAsync(a, F, sizeof(double) * nF, cudaMemcpyHostToDevice, p->stream));
     Fd = a;
   }
-  {
+  if (p->symmetry == HP_REAL) {
+    HP_CHECK(real_backward_rows(p, Fd, fd, nbatch, p->stream));
+  } else {
+    const double* psi = real_psi(p, &st);
+    if (st) return st;
+    double2* SF = (double2*)p->ws_get("real.S", sizeof(double2) * (size_t)D * D * N * nbatch, &st);
+    if (st) return st;
     ProfScope _ps(p, "real.bwd", p->stream);
     const long long nt = (long long)D * D * N * nbatch;
     k_real_bwd_beta<<<(unsigned)((nt + 127) / 128), 128, 0, p->stream>>>(B, nbatch, Fd, psi, SF);
@@ -349,6 +364,116 @@ __global__ void k_cplx_to_real(int B, int nb, const double2* __restrict__ Xc, do
     }
   }
   Xr[t] = acc;
+}
+
+// ------------------------------------- transforms through complex rows ----
+// F_c(m, n) of a real function for any m from the stored rows (m >= 0):
+// F_c(-m, -n) = (-1)^(m-n) conj F_c(m, n).
+__device__ __forceinline__ double2 row_coeff(const RowLayout& L, const double2* X, int nb, int b, int l, int m, int n) {
+  const int am = abs(m), sn = m < 0 ? -n : n, an = abs(n);
+  const long long row = L.seg[am * (2 * L.lmax + 1) + sn + L.lmax] + l - (am > an ? am : an);
+  double2 v = X[row * nb + b];
+  if (m < 0) {
+    const double sg = ((m - n) & 1) ? -1.0 : 1.0;
+    v = make_double2(sg * v.x, -sg * v.y);
+  }
+  return v;
+}
+
+// F_r = Re T F_c T^H, [row][nb] -> F(m, n, l, b); tiles of 32 full indices x 32
+// functions (lanes read along the functions and write along the full index)
+__global__ void k_rows_to_real(RowLayout L, int nb, const double2* __restrict__ X, double* __restrict__ F) {
+  __shared__ double tile[32][33];
+  const int lmax = L.lmax, D = 2 * lmax + 1, per = D * D * (lmax + 1);
+  const int fi0 = blockIdx.x * 32, b0 = blockIdx.y * 32;
+  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+    const int fi = fi0 + k, b = b0 + threadIdx.x;
+    const int l = fi / (D * D), m = fi % D - lmax, n = fi / D % D - lmax;
+    double acc = 0.0;
+    if (fi < per && b < nb && abs(m) <= l && abs(n) <= l) {
+      for (int ip = 0; ip < (m == 0 ? 1 : 2); ++ip) {
+        const int p = ip ? -m : m;
+        const double2 a = t_entry(m, p);
+        for (int iq = 0; iq < (n == 0 ? 1 : 2); ++iq) {
+          const int q = iq ? -n : n;
+          const double2 c = t_entry(n, q);                 // conjugated below
+          const double2 x = row_coeff(L, X, nb, b, l, p, q);
+          const double2 ax = make_double2(a.x * x.x - a.y * x.y, a.x * x.y + a.y * x.x);
+          acc += ax.x * c.x + ax.y * c.y;                  // Re(a x conj(c))
+        }
+      }
+    }
+    tile[k][threadIdx.x] = acc;
+  }
+  __syncthreads();
+  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+    const int fi = fi0 + threadIdx.x, b = b0 + k;
+    if (fi < per && b < nb) F[fi + (long long)per * b] = tile[threadIdx.x][k];
+  }
+}
+
+// F_c = T^H F_r T, F(m, n, l, b) -> [row][nb] (m >= 0); tiles of 32 kept entries
+// in full-layout order x 32 functions
+__global__ void k_real_to_rows(RowLayout L, const int2* __restrict__ fg, int nb, const double* __restrict__ F,
+                               double2* __restrict__ X) {
+  __shared__ double2 tile[32][33];
+  const int lmax = L.lmax, D = 2 * lmax + 1, per = D * D * (lmax + 1), nrows = (int)L.nrows;
+  const int e0 = blockIdx.x * 32, b0 = blockIdx.y * 32, e = e0 + threadIdx.x;
+  int m = 0, n = 0, base = 0;
+  if (e < nrows) {
+    const char4 q = L.rows[fg[e].y];
+    m = q.y;
+    n = q.z;
+    base = D * D * q.x;
+  }
+  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+    double2 acc = make_double2(0.0, 0.0);
+    if (e < nrows && b0 + k < nb) {
+      const double* Fb = F + (long long)per * (b0 + k) + base;
+      for (int ip = 0; ip < (m == 0 ? 1 : 2); ++ip) {
+        const int p = ip ? -m : m;
+        const double2 a = t_entry(p, m);                   // conjugated below
+        for (int iq = 0; iq < (n == 0 ? 1 : 2); ++iq) {
+          const int q = iq ? -n : n;
+          const double2 c = t_entry(q, n);
+          const double v = Fb[(p + lmax) + D * (q + lmax)];
+          acc.x += v * (a.x * c.x + a.y * c.y);
+          acc.y += v * (a.x * c.y - a.y * c.x);
+        }
+      }
+    }
+    tile[k][threadIdx.x] = acc;
+  }
+  __syncthreads();
+  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+    const int b = b0 + threadIdx.x;
+    if (e0 + k < nrows && b < nb) X[(long long)fg[e0 + k].y * nb + b] = tile[threadIdx.x][k];
+  }
+}
+
+static int real_forward_rows(hp_plan* p, const double* f, double* F, int nb, cudaStream_t s) {
+  int st = HP_OK;
+  double2* rows = (double2*)p->ws_get("real.rows", sizeof(double2) * (size_t)p->nrows * nb, &st);
+  if (st) return st;
+  HP_CHECK(hp_so3_forward64(p, f, rows, nb, s));
+  ProfScope _ps(p, "real.fwd", s);
+  const int per = p->D * p->D * p->B;
+  k_rows_to_real<<<dim3((per + 31) / 32, (nb + 31) / 32), dim3(32, 8), 0, s>>>(p->layout(), nb, rows, F);
+  HP_CUDA_TRY(cudaGetLastError());
+  return HP_OK;
+}
+
+static int real_backward_rows(hp_plan* p, const double* F, double* f, int nb, cudaStream_t s) {
+  int st = HP_OK;
+  double2* rows = (double2*)p->ws_get("real.rows", sizeof(double2) * (size_t)p->nrows * nb, &st);
+  if (st) return st;
+  {
+    ProfScope _ps(p, "real.bwd", s);
+    k_real_to_rows<<<dim3((unsigned)((p->nrows + 31) / 32), (nb + 31) / 32), dim3(32, 8), 0, s>>>(p->layout(), p->fgather, nb,
+                                                                                               F, rows);
+    HP_CUDA_TRY(cudaGetLastError());
+  }
+  return hp_so3_backward64(p, rows, f, nb, s);
 }
 
 extern "C" int hp_fftSO3_real_prod(hp_plan* p, const double* F, const double* G, double* FG, int batch, int mem) {
