@@ -275,6 +275,22 @@ template <typename T> struct PlaneCfg;   // MINB: blocks per SM of the persisten
 template <> struct PlaneCfg<double> { static constexpr int C = 1; static constexpr int NT = 128; static constexpr int MINB = 2; };
 template <> struct PlaneCfg<float> { static constexpr int C = 2; static constexpr int NT = 256; static constexpr int MINB = 2; };
 
+// The model's constants in the pass's precision, converted on the host: the
+// arithmetic reads them from the constant bank instead of holding registers
+// (four RK4 passes at B = 11, 22^3, FP32: 1.34 -> 1.23 ms; B = 12, 24^3, FP64:
+// 0.766 -> 0.735).
+template <typename T> struct PlanePrm {
+  T half_L, dx, tp, lie, b[3], g[3];
+  __host__ __device__ PlanePrm(const DerivParams& q, int N) {
+    const T L = (T)q.L;
+    half_L = L / 2;
+    dx = L / (T)N;
+    tp = (T)(2.0 * M_PI / q.L);
+    lie = (T)q.lie;
+    for (int i = 0; i < 3; ++i) { b[i] = (T)q.b[i]; g[i] = (T)q.gyro[i]; }
+  }
+};
+
 // Resident blocks per SM that the registers are held to.  The pass waits for
 // its own barriers and FP64 chains more than for anything it could compute, so
 // more blocks pay even where a few registers spill; shared memory (C + 2 F
@@ -311,7 +327,7 @@ __device__ __forceinline__ void plane_body(const RowLayout& L, const PlaneTile t
                                            const c2<TIN>* __restrict__ Fev, const c2<T>* __restrict__ P3,
                                            const c2<T>* __restrict__ Gl, const double2* __restrict__ F0, double a,
                                            double2* __restrict__ out, double2* __restrict__ acc, double bacc,
-                                           const DerivParams& prm, c2<T>* __restrict__ out32, unsigned char* smraw) {
+                                           const PlanePrm<T>& prm, c2<T>* __restrict__ out32, unsigned char* smraw) {
   using C = c2<T>;
   constexpr int CT = PlaneCfg<T>::C;
   constexpr int PS = N * (N + 1);
@@ -324,8 +340,7 @@ __device__ __forceinline__ void plane_body(const RowLayout& L, const PlaneTile t
 
   const long long pbase = (long long)k3 * N * N;  // plane offset inside a row
   const int tid = threadIdx.x, nth = blockDim.x;
-  const T Ll = (T)prm.L;
-  const T tp = (T)(2.0 * M_PI / prm.L);
+  const T tp = prm.tp;
   const T inv_n2 = (T)1 / (T)(N * N);
 
   // ---- S1: load F rows n0-1 .. n0+cnt and P3 rows n0 .. n0+cnt-1 ----
@@ -455,19 +470,21 @@ __device__ __forceinline__ void plane_body(const RowLayout& L, const PlaneTile t
   constexpr int H = N / 2;
   const int h = tid & 1, pr = tid >> 1, npr = nth >> 1;
   const T d3 = HAS_P3 ? tp * (T)kappa_first(k3, N) : (T)0;
-  const T b1 = (T)prm.b[0], b2 = (T)prm.b[1], b3 = (T)prm.b[2];
-  const T g1 = (T)prm.gyro[0], g2 = (T)prm.gyro[1], g3 = (T)prm.gyro[2];
+  T b1 = prm.b[0], b2 = prm.b[1], b3 = prm.b[2];
+  T g1 = prm.g[0], g2 = prm.g[1], g3 = prm.g[2];
+  if constexpr (sizeof(T) == 4 && N > 30)   // registers to spare at two blocks per SM: keep them there
+    asm volatile("" : "+f"(b1), "+f"(b2), "+f"(b3), "+f"(g1), "+f"(g2), "+f"(g3));
   for (int it = pr; it < tl.cnt * N * 2; it += npr) {   // both lanes of a pair hold the same item
     const int kind = it / (tl.cnt * N);
     const int c = (it / N) % tl.cnt;
     const int j1 = it % N;
-    const T x1 = -Ll / 2 + Ll * (T)j1 / (T)N;
+    const T x1 = prm.dx * (T)j1 - prm.half_L;
     const C* f0 = sF + (c + 1) * PS;
     const C* fm = sF + c * PS;
     const C* fp = sF + (c + 2) * PS;
     const C* pp = sP + c * PS;
     const int n = tl.n0 + c, l = tl.l;
-    const T lie = (T)prm.lie;
+    const T lie = prm.lie;
     const T ap = lie * sqrt((T)((l - n) * (l + n + 1))), am = lie * sqrt((T)((l + n) * (l - n + 1)));
     C x[H];
     if (kind == 0) {
@@ -475,7 +492,7 @@ __device__ __forceinline__ void plane_body(const RowLayout& L, const PlaneTile t
 #pragma unroll
       for (int j = 0; j < H; ++j) {
         const int j2 = 2 * j + h;
-        const T x2 = -Ll / 2 + Ll * (T)j2 / (T)N;
+        const T x2 = prm.dx * (T)j2 - prm.half_L;
         const int o = j2 * (N + 1) + j1;
         const C vp = fp[o], vm = fm[o];
         C y;
@@ -503,7 +520,7 @@ __device__ __forceinline__ void plane_body(const RowLayout& L, const PlaneTile t
 #pragma unroll
       for (int j = 0; j < H; ++j) {
         const int j2 = 2 * j + h;
-        const T x2 = -Ll / 2 + Ll * (T)j2 / (T)N;
+        const T x2 = prm.dx * (T)j2 - prm.half_L;
         const int o = j2 * (N + 1) + j1;
         C y = (b2 * x2) * f0[o];
         if (HAS_P3) y = y - (g2 * x1) * pp[o];
@@ -525,7 +542,7 @@ __device__ __forceinline__ void plane_body(const RowLayout& L, const PlaneTile t
 #pragma unroll
       for (int j = 0; j < H; ++j) {
         const int j2 = 2 * j + h;
-        const T x2 = -Ll / 2 + Ll * (T)j2 / (T)N;
+        const T x2 = prm.dx * (T)j2 - prm.half_L;
         const int o = j2 * (N + 1) + j1;
         C y = (b1 * x1) * f0[o];
         if (HAS_P3) y = y - (g1 * x2) * pp[o];
@@ -619,7 +636,7 @@ __global__ void __launch_bounds__(PlaneCfg<T>::NT, (plane_minb<N, T, HAS_P3>()))
                                                   const double2* __restrict__ F0, double a,
                                                   double2* __restrict__ out,
                                                   double2* __restrict__ acc, double bacc,
-                                                  DerivParams prm, c2<T>* __restrict__ out32 = nullptr) {
+                                                  PlanePrm<T> prm, c2<T>* __restrict__ out32 = nullptr) {
   extern __shared__ __align__(16) unsigned char smraw[];
   plane_body<N, T, HAS_P3, TIN>(L, tiles[blockIdx.x], HAS_P3 ? (int)blockIdx.y : 0, Fev, P3, Gl, F0, a, out, acc, bacc,
                                 prm, out32, smraw);
@@ -638,7 +655,7 @@ template <int N, typename T>
 __device__ __noinline__ void plane_item(const PlaneJob& jb, const PlaneTile tl, int k3, unsigned char* smraw) {
   using C = c2<T>;
   plane_body<N, T, true, T>(jb.L, tl, k3, (const C*)jb.Fev, (const C*)jb.P3, (const C*)jb.G, jb.F0, jb.a, jb.out,
-                            jb.acc, jb.bacc, jb.prm, (C*)jb.out32, smraw);
+                            jb.acc, jb.bacc, PlanePrm<T>(jb.prm, N), (C*)jb.out32, smraw);
 }
 
 template <typename T>
@@ -860,14 +877,14 @@ static int run_deriv_N(hp_plan* p, const double2* Fev, const double2* F0, double
   ProfScope _ps(p, "deriv.plane", s);
   if (p3 && Fc) {
     HP_CUDA_TRY(cudaFuncSetAttribute(k_plane<N, T, true, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_plane<N, T, true, T><<<grid, PlaneCfg<T>::NT, smem, s>>>(L, dt, Fc, P3, G, F0, a, out, acc, bacc, prm,
+    k_plane<N, T, true, T><<<grid, PlaneCfg<T>::NT, smem, s>>>(L, dt, Fc, P3, G, F0, a, out, acc, bacc, PlanePrm<T>(prm, N),
                                                                 (C*)(mixed3 ? out32 : nullptr));
   } else if (p3) {
     HP_CUDA_TRY(cudaFuncSetAttribute(k_plane<N, T, true, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_plane<N, T, true, double><<<grid, PlaneCfg<T>::NT, smem, s>>>(L, dt, Fev, P3, G, F0, a, out, acc, bacc, prm);
+    k_plane<N, T, true, double><<<grid, PlaneCfg<T>::NT, smem, s>>>(L, dt, Fev, P3, G, F0, a, out, acc, bacc, PlanePrm<T>(prm, N));
   } else {
     HP_CUDA_TRY(cudaFuncSetAttribute(k_plane<N, T, false, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_plane<N, T, false, double><<<grid, PlaneCfg<T>::NT, smem, s>>>(L, dt, Fev, P3, G, F0, a, out, acc, bacc, prm);
+    k_plane<N, T, false, double><<<grid, PlaneCfg<T>::NT, smem, s>>>(L, dt, Fev, P3, G, F0, a, out, acc, bacc, PlanePrm<T>(prm, N));
   }
   HP_CUDA_TRY(cudaGetLastError());
   return HP_OK;
@@ -1297,10 +1314,10 @@ static int noalloc_N(hp_plan* p, const double2* Ffull, double2* dFfull, unsigned
   dim3 grid((unsigned)ntiles, p3 ? N : 1);
   if (p3) {
     HP_CUDA_TRY(cudaFuncSetAttribute(k_plane<N, T, true, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_plane<N, T, true, double><<<grid, PlaneCfg<T>::NT, smem, s>>>(L, tiles, Fi, P3, G, nullptr, 1.0, dFi, nullptr, 0.0, prm);
+    k_plane<N, T, true, double><<<grid, PlaneCfg<T>::NT, smem, s>>>(L, tiles, Fi, P3, G, nullptr, 1.0, dFi, nullptr, 0.0, PlanePrm<T>(prm, N));
   } else {
     HP_CUDA_TRY(cudaFuncSetAttribute(k_plane<N, T, false, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_plane<N, T, false, double><<<grid, PlaneCfg<T>::NT, smem, s>>>(L, tiles, Fi, P3, G, nullptr, 1.0, dFi, nullptr, 0.0, prm);
+    k_plane<N, T, false, double><<<grid, PlaneCfg<T>::NT, smem, s>>>(L, tiles, Fi, P3, G, nullptr, 1.0, dFi, nullptr, 0.0, PlanePrm<T>(prm, N));
   }
   HP_CUDA_TRY(cudaGetLastError());
   return hp_internal_to_full(p, dFi, dFfull, s);
