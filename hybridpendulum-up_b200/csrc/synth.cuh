@@ -270,21 +270,21 @@ __global__ void __launch_bounds__(RealSynthCfg<B, T>::NT, 1)
   if (al16) bulk_wait_all();   // shared memory must outlive the bulk copies reading it
 }
 
-// (m, n >= 0) pairs: row starts of (m, n) and (m, -n), length of their l-run,
-// m and n; longest runs first
+// Entry q < B^2: the pair (m, n >= 0) with row starts of (m, n) and (m, -n),
+// length of their l-run, m and n; longest runs first.  The (max(m, n) + 1)^2
+// pairs up to max(m, n) come before all others, so q gives its pair in closed
+// form, and the table is built on the device in the buffer of the d table:
+// a new plan's first synthesis needs no allocation, copy and wait for it.
 template <int B>
-static int build_real_pairs(hp_plan* p, int2* dpairs) {
-  const int lmax = B - 1, D = 2 * lmax + 1;
-  std::vector<int2> v;
-  for (int lmin = 0; lmin < B; ++lmin)
-    for (int m = 0; m <= lmin; ++m)
-      for (int n = 0; n <= lmin; ++n) {
-        if (std::max(m, n) != lmin) continue;
-        const int sp = p->h_seg[(size_t)m * D + n + lmax], sn = p->h_seg[(size_t)m * D - n + lmax];
-        v.push_back(make_int2((int)((unsigned)sp | ((unsigned)sn << 16)), (B - lmin) | (m << 8) | (n << 16)));
-      }
-  HP_CUDA_TRY(cudaMemcpy(dpairs, v.data(), sizeof(int2) * v.size(), cudaMemcpyHostToDevice));
-  return HP_OK;
+__global__ void k_node_pairs(RowLayout L, int2* __restrict__ out) {
+  constexpr int lmax = B - 1, D = 2 * lmax + 1;
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= B * B) return;
+  int lmin = 0;
+  while ((lmin + 1) * (lmin + 1) <= q) ++lmin;
+  const int r = q - lmin * lmin, m = min(r, lmin), n = r < lmin ? lmin : r - lmin;
+  const int* seg = L.seg + (m - L.m_lo) * D + lmax;
+  out[q] = make_int2((int)((unsigned)seg[n] | ((unsigned)seg[-n] << 16)), (B - lmin) | (m << 8) | (n << 16));
 }
 
 template <int B, typename T>
@@ -292,24 +292,20 @@ int synth_real_launch(hp_plan* p, const c2<T>* Fp, T* f, cudaStream_t s) {
   using Cfg = RealSynthCfg<B, T>;
   constexpr int NN = Cfg::NN, P = Cfg::P, NG = (B + NN - 1) / NN;
   int st = HP_OK;
-  bool have = false;
-  for (auto& kv : p->ws) if (kv.first == "tf.pairs_n") have = true;
-  int2* dpairs = (int2*)p->ws_get("tf.pairs_n", sizeof(int2) * B * B, &st);
-  if (st) return st;
-  if (!have) {
-    st = build_real_pairs<B>(p, dpairs);
-    if (st) return st;
-  }
-  // (2l+1) d at the nodes as [group][row][NN]
+  // (2l+1) d at the nodes as [group][row][NN], then the pairs (8-byte aligned)
   const char* key = sizeof(T) == 8 ? "tf.sdn64" : "tf.sdn32";
-  have = false;
+  bool have = false;
   for (auto& kv : p->ws) if (kv.first == key) have = true;
-  const long long n = (long long)NG * p->nrows * NN;
-  T* dtab = (T*)p->ws_get(key, sizeof(T) * n, &st);
+  const long long n = (long long)NG * p->nrows * NN, nd = (sizeof(T) * n + 15) / 16 * 16;
+  char* tab = (char*)p->ws_get(key, nd + sizeof(int2) * B * B, &st);
   if (st) return st;
+  T* dtab = (T*)tab;
+  int2* dpairs = (int2*)(tab + nd);
   if (!have) {
     k_sd_table<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
         p->layout(), sizeof(T) == 8 ? (const T*)(const void*)p->wig64 : (const T*)(const void*)p->wig32, dtab, NN, NG);
+    HP_CUDA_TRY(cudaGetLastError());
+    k_node_pairs<B><<<(B * B + 127) / 128, 128, 0, s>>>(p->layout(), dpairs);
     HP_CUDA_TRY(cudaGetLastError());
   }
   constexpr size_t smem = (size_t)Cfg::bytes(NN, P);
