@@ -757,8 +757,6 @@ template <typename T> static size_t plane_smem(int N, bool p3) {
 }
 
 
-// k_local with the widest omega tile (32/16/8/4 points) whose group tile and
-// tap weights fit 110 KB of shared memory (the m = 0 group has (lmax+1)^2 rows).
 template <typename T, int W, typename TIN>
 static int local_w_launch(hp_plan* p, const c2<TIN>* F, c2<T>* G, const c2<T>* Gx, const DerivParams& prm,
                           cudaStream_t s) {
@@ -781,12 +779,27 @@ static int local_w_launch(hp_plan* p, const c2<TIN>* F, c2<T>* G, const c2<T>* G
   return HP_OK;
 }
 
+// k_local with the widest omega tile (32/16/8/4 points) whose group tile and
+// tap weights fit 110 KB of shared memory (the m = 0 group has (lmax+1)^2 rows)
+// and that leaves about two blocks per SM, or whose half would leave threads of
+// the widest group without a row: on small grids a block walks its rows in a
+// serial chain while SMs idle.  RK4 step with density, us, widest that fits /
+// this: FP32 2-D B = 8, 16^2 69.7 / 61.5, B = 12, 16^2 117 / 95, B = 16, 16^2
+// 178 / 145; FP64 B = 16, 16^2 202 / 193.  The lines: 256 blocks of 16 points
+// (FP64 B = 16, 16^2) lose to 512 of 8, 288 (B = 8, 24^2) win, 86.5 against 88.6;
+// half the threads idle at 8 points for B = 4 (3-D, 8^3: 73.6 at 16, 77.5 at 8).
 template <typename T, typename TIN = double>
 static int launch_local(hp_plan* p, const c2<TIN>* F, c2<T>* G, const c2<T>* Gx, const DerivParams& prm,
                         cudaStream_t s) {
   constexpr size_t budget = 110 * 1024;
-  if (sizeof(T) == 4 && local_smem<T>(p, 32) <= budget) return local_w_launch<T, 32, TIN>(p, F, G, Gx, prm, s);
-  if (local_smem<T>(p, 16) <= budget) return local_w_launch<T, 16, TIN>(p, F, G, Gx, prm, s);
+  constexpr long long min_blocks = 280;
+  const int rmax = (p->lmax + 1) * (p->lmax + 1);
+  const auto take = [&](int W) {
+    return local_smem<T>(p, W) <= budget &&
+           ((p->nx + W - 1) / W * p->nm >= min_blocks || rmax * (W / 2) < 256);
+  };
+  if (sizeof(T) == 4 && take(32)) return local_w_launch<T, 32, TIN>(p, F, G, Gx, prm, s);
+  if (take(16)) return local_w_launch<T, 16, TIN>(p, F, G, Gx, prm, s);
   if (local_smem<T>(p, 8) <= budget) return local_w_launch<T, 8, TIN>(p, F, G, Gx, prm, s);
   if (local_smem<T>(p, 4) <= (size_t)200 * 1024) return local_w_launch<T, 4, TIN>(p, F, G, Gx, prm, s);
   hp_set_error("gravity pass tiles exceed shared memory for this bandlimit");

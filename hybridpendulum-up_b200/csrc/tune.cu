@@ -3,8 +3,8 @@
 // loaded from a text file.
 //
 // The knobs are the runtime launch shapes of the two transforms:
-//   synth_pt    omega points per beta-stage item of the synthesis (FP32
-//               plans: 1, 2 or 4; an item then holds an NB x PT output tile)
+//   synth_pt    no effect now (it shaped an earlier synthesis kernel); kept in
+//               the interface and in the file, where 1, 2 and 4 are accepted
 //   synth_waves resident waves of synthesis blocks (4, 8 or 16): how many
 //               omega chunks each block walks through
 //   tc_waves    waves of tensor-core CTAs of the forward beta contraction
