@@ -781,20 +781,24 @@ static int local_w_launch(hp_plan* p, const c2<TIN>* F, c2<T>* G, const c2<T>* G
 
 // k_local with the widest omega tile (32/16/8/4 points) whose group tile and
 // tap weights fit 110 KB of shared memory (the m = 0 group has (lmax+1)^2 rows)
-// and that leaves about two blocks per SM, or whose half would leave threads of
-// the widest group without a row: on small grids a block walks its rows in a
-// serial chain while SMs idle.  RK4 step with density, us, widest that fits /
-// this: FP32 2-D B = 8, 16^2 69.7 / 61.5, B = 12, 16^2 117 / 95, B = 16, 16^2
-// 178 / 145; FP64 B = 16, 16^2 202 / 193.  The lines: 256 blocks of 16 points
-// (FP64 B = 16, 16^2) lose to 512 of 8, 288 (B = 8, 24^2) win, 86.5 against 88.6;
-// half the threads idle at 8 points for B = 4 (3-D, 8^3: 73.6 at 16, 77.5 at 8).
+// and that leaves enough blocks, or whose half would leave threads of the widest
+// group without a row: on small grids a block walks its rows in a serial chain
+// while SMs idle.  RK4 step with density, us, widest that fits / this: FP32 2-D
+// B = 8, 16^2 69.7 / 61.5, B = 12, 16^2 117 / 95, B = 16, 16^2 178 / 145; FP64
+// B = 16, 16^2 202 / 193.  The lines, us: 2-D, 16 points, 256 blocks (FP64 B = 16,
+// 16^2) 202 against 193 at 8, 288 (B = 8, 24^2) 86.5 against 88.6; 32 points (the
+// FP64 state is read: 16 are still 256 bytes), 288 blocks (FP32 B = 16, 24^2)
+// 331 against 298 at 16, 512 (32^2) 535 against 508.  3-D (three passes share the
+// step, FP32 input): 512 blocks of 32 (FP32 B = 4, 16^3) 88 against 98 at 16, 128
+// (B = 8, 8^3) 110.7 at 32 and 16, 111.8 at 8.  Half the threads idle at 8 points
+// for B = 4 (3-D, 8^3: 73.6 at 16, 77.5 at 8).
 template <typename T, typename TIN = double>
 static int launch_local(hp_plan* p, const c2<TIN>* F, c2<T>* G, const c2<T>* Gx, const DerivParams& prm,
                         cudaStream_t s) {
   constexpr size_t budget = 110 * 1024;
-  constexpr long long min_blocks = 280;
   const int rmax = (p->lmax + 1) * (p->lmax + 1);
   const auto take = [&](int W) {
+    const long long min_blocks = p->ndim == 3 ? 148 : W == 32 ? 592 : 280;
     return local_smem<T>(p, W) <= budget &&
            ((p->nx + W - 1) / W * p->nm >= min_blocks || rmax * (W / 2) < 256);
   };
