@@ -5,7 +5,9 @@
 // After one eager warm-up step (which sizes every workspace), two steps of the
 // whole batch are captured into one CUDA graph and replayed: the state
 // buffers ping-pong with period two for every method, so a two-step graph
-// starts and ends on the same buffers.  An odd remainder runs eagerly.
+// starts and ends on the same buffers.  An odd remainder runs eagerly.  The
+// graph holds addresses of the plans' workspaces: another call on a member's
+// plan that grows or releases one of those drops the graph.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -42,6 +44,7 @@ struct hp_batch {
   int method = -1;
   std::vector<double2*> capF;               // each member's F at capture
   std::vector<int> capF32;                  // and its FP32-copy state: valid * 2 + current slot
+  std::vector<long long> cap_freed;         // each plan's count of freed workspace buffers at capture
   long long graph_launches = 0;
 };
 
@@ -152,7 +155,17 @@ bool at_capture_buffers(const hp_batch* b) {
   return true;
 }
 
+// The graph's kernels read and write workspace buffers of the plans: no plan
+// has freed one since the capture began.
+bool workspaces_in_place(const hp_batch* b) {
+  for (size_t i = 0; i < b->plans.size(); ++i)
+    if (b->plans[i]->ws_freed != b->cap_freed[i]) return false;
+  return true;
+}
+
 int capture(hp_batch* b, double dt, int method) {
+  b->cap_freed.clear();
+  for (auto p : b->plans) b->cap_freed.push_back(p->ws_freed);
   b->capF.clear();
   b->capF32.clear();
   for (auto s : b->st) {
@@ -257,7 +270,7 @@ extern "C" int hp_batch_step(hp_batch* b, double dt, int method, int nsteps) {
   if (!std::isfinite(dt)) { hp_set_error("dt must be finite"); return HP_ERR_INVALID; }
   for (auto p : b->plans)
     if (p->prof_on) { hp_set_error("disable plan profiling before batched steps"); return HP_ERR_INVALID; }
-  if (b->exec && (dt != b->dt || method != b->method)) drop_graph(b);
+  if (b->exec && (dt != b->dt || method != b->method || !workspaces_in_place(b))) drop_graph(b);
   BT_CHECK(use_streams(b, true));
   int st = HP_OK;
   int done = 0;
@@ -269,13 +282,14 @@ extern "C" int hp_batch_step(hp_batch* b, double dt, int method, int nsteps) {
       if (e != cudaSuccess) { hp_set_error(cudaGetErrorString(e)); st = HP_ERR_CUDA; }
     }
     if (st == HP_OK) st = capture(b, dt, method);
+    if (st == HP_OK && !workspaces_in_place(b)) drop_graph(b);   // a buffer moved within the captured steps
   }
   if (st == HP_OK && b->exec) {
     if (!at_capture_buffers(b) && nsteps - done >= 1) {
       st = batch_step(b, dt, method);
       ++done;
     }
-    while (st == HP_OK && nsteps - done >= 2 && at_capture_buffers(b)) {
+    while (st == HP_OK && nsteps - done >= 2 && at_capture_buffers(b) && workspaces_in_place(b)) {
       const cudaError_t e = cudaGraphLaunch(b->exec, b->origin);
       if (e != cudaSuccess) { hp_set_error(cudaGetErrorString(e)); st = HP_ERR_CUDA; break; }
       ++b->graph_launches;

@@ -78,6 +78,7 @@ extern "C" const char* hp_last_error(void) { return g_err.c_str(); }
 void hp_plan::ws_release(const char* name) {
   for (auto& kv : ws)
     if (kv.first == name && kv.second.p) {
+      ++ws_freed;
       hp_dev_free(kv.second.p);
       kv.second = Buf{};
     }
@@ -87,6 +88,7 @@ void* hp_plan::ws_get(const char* name, size_t bytes, int* status) {
   for (auto& kv : ws) {
     if (kv.first == name) {
       if (kv.second.bytes >= bytes) return kv.second.p;
+      if (kv.second.p) ++ws_freed;
       hp_dev_free(kv.second.p);
       kv.second = Buf{};
       void* q = nullptr;

@@ -92,6 +92,9 @@ struct hp_plan {
   std::vector<std::pair<std::string, Buf>> ws;
   void* ws_get(const char* name, size_t bytes, int* status);
   void ws_release(const char* name);   // frees a workspace buffer (re-created on demand)
+  // workspace buffers freed so far (grown or released): what holds addresses of
+  // the workspace, a captured graph above all, is stale once this has moved
+  long long ws_freed = 0;
 
   RowLayout layout() const {
     RowLayout L;
