@@ -17,6 +17,7 @@
 // FP32 0.49 / 0.16.  Where both forms exist the one-pass kernel is faster (24^3,
 // B = 12 FP32: 0.48 against 0.66 ms, B = 15 FP64: 1.93 against 2.58).
 #pragma once
+#include "row_groups.hpp"
 
 // G of one chunk of omega points: half of the 126 MB L2
 constexpr long long kSynthG = 64LL << 20;
@@ -66,11 +67,11 @@ __global__ void __launch_bounds__(128) k_synth_beta(long long nx, const c2<T>* _
   // the warp's table rows (whole groups of four: the rows past the run multiply
   // zero coefficients) go to shared memory in one go; read from L2 a sector at
   // a time as the betas advance, they were the stall of three issues in four
-  T* d = reinterpret_cast<T*>(smraw) + (threadIdx.x >> 5) * ((B + 3) / 4 * 4 * DS);
+  T* d = reinterpret_cast<T*>(smraw) + (threadIdx.x >> 5) * (rows_copied(B) * DS);
   {
     constexpr int EPP = 16 / (int)sizeof(T);
     const T* dsrc = dtab + (size_t)s * DS;
-    for (int e = lane; e < (len + 3) / 4 * 4 * DS / EPP; e += 32) cp_async<16>(d + e * EPP, dsrc + e * EPP, true);
+    for (int e = lane; e < rows_copied(len) * DS / EPP; e += 32) cp_async<16>(d + e * EPP, dsrc + e * EPP, true);
   }
   const long long wl = (long long)blockIdx.x * 32 + lane;
   const C* src = Fp + (size_t)s * nx + w0 + wl;
@@ -226,12 +227,12 @@ __global__ void __launch_bounds__(Synth2Cfg<B, T, CPLX>::NT, Synth2Cfg<B, T, CPL
   }
 }
 
-// (2l+1) d^l_mn(beta_b) as [row][DS], zero beyond b = 2B and in B more rows
-// (k_synth_beta reads whole groups of four rows)
+// (2l+1) d^l_mn(beta_b) as [row][DS], zero beyond b = 2B and in the kRowPad rows
+// behind the last one (k_synth_beta reads whole groups of rows)
 template <typename T>
 __global__ void k_dsyn_table(RowLayout L, const T* __restrict__ wig, int DS, T* __restrict__ out) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= (L.nrows + L.B) * DS) return;
+  if (t >= (L.nrows + kRowPad) * DS) return;
   const long long r = t / DS;
   const int b = (int)(t % DS);
   out[t] = r < L.nrows && b < 2 * L.B ? (T)(2 * L.rows[r].x + 1) * wig[(size_t)b * L.nrows + r] : (T)0;
@@ -256,10 +257,10 @@ int synth2_launch(hp_plan* p, const c2<T>* Fp, void* f, long long nx, cudaStream
   const char* dkey = sizeof(T) == 8 ? "tf.dsyn64" : "tf.dsyn32";
   have = false;
   for (auto& kv : p->ws) if (kv.first == dkey) have = true;
-  T* dtab = (T*)p->ws_get(dkey, sizeof(T) * (p->nrows + B) * DS, &st);
+  T* dtab = (T*)p->ws_get(dkey, sizeof(T) * (p->nrows + kRowPad) * DS, &st);
   if (st) return st;
   if (!have) {
-    const long long n = (p->nrows + B) * DS;
+    const long long n = (p->nrows + kRowPad) * DS;
     k_dsyn_table<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
         p->layout(), sizeof(T) == 8 ? (const T*)(const void*)p->wig64 : (const T*)(const void*)p->wig32, DS, dtab);
     HP_CUDA_TRY(cudaGetLastError());
@@ -276,7 +277,7 @@ int synth2_launch(hp_plan* p, const c2<T>* Fp, void* f, long long nx, cudaStream
     const long long nw = std::min(nwc, nx - w0);
     {
       ProfScope _ps(p, "tf.synth.beta", s);
-      constexpr size_t dsm = 4 * sizeof(T) * (size_t)((B + 3) / 4 * 4 * DS);
+      constexpr size_t dsm = 4 * sizeof(T) * (size_t)(rows_copied(B) * DS);
       HP_CUDA_TRY(cudaFuncSetAttribute(k_synth_beta<B, T, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm));
       k_synth_beta<B, T, CPLX><<<dim3((unsigned)((nw + 31) / 32), (unsigned)((NPAIR + 3) / 4)), 128, dsm, s>>>(
           nx, Fp, dtab, dpairs, NPAIR, G, w0, nw);
