@@ -24,8 +24,43 @@ using namespace hp;
 constexpr int kProdR = 6;                     // outputs per thread of the convolution
 constexpr long long kProdH = 256LL << 20;     // bytes of H per launch
 
+__device__ __forceinline__ bool finite2(double2 a) { return isfinite(a.x) && isfinite(a.y); }
+
+// What the infinite and NaN entries of SF add to H, each where it meets SG and
+// nowhere else.  Called by blocks that have any, after their other sums.
+__device__ __noinline__ void prod_conv_nonfinite(int B, const double* __restrict__ dj, const double2* __restrict__ Fb,
+                                                 double2* sf, const double2* sg, double2* Hj) {
+  const int lmax = B - 1, D = 2 * lmax + 1, SW = D + 2 * kProdR;
+  for (int e = threadIdx.x; e < D * D; e += blockDim.x) {
+    const int mi = e % D, ni = e / D, l0 = max(abs(mi - lmax), abs(ni - lmax));
+    double2 a = make_double2(0.0, 0.0);
+    for (int l = l0; l < B; ++l) {
+      const long long q = e + (long long)D * D * l;
+      const double w = (2 * l + 1) * dj[q];
+      a.x = fma(w, Fb[q].x, a.x); a.y = fma(w, Fb[q].y, a.y);
+    }
+    sf[mi * D + ni] = finite2(a) ? make_double2(0.0, 0.0) : a;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < D * D; e += blockDim.x) {
+    const int mi = e % D, ni = e / D;
+    double2 h = Hj[e];
+    for (int m1i = max(0, mi - lmax); m1i <= min(D - 1, mi + lmax); ++m1i)
+      for (int n1i = max(0, ni - lmax); n1i <= min(D - 1, ni + lmax); ++n1i) {
+        const double2 f = sf[m1i * D + n1i];
+        if (f.x == 0.0 && f.y == 0.0) continue;
+        const double2 g = sg[(mi - m1i + lmax) * SW + kProdR + ni - n1i + lmax];
+        h.x = fma(f.x, g.x, fma(-f.y, g.y, h.x));
+        h.y = fma(f.x, g.y, fma(f.y, g.x, h.y));
+      }
+    Hj[e] = h;
+  }
+}
+
 // Block = (node j, product b).  SG rows have R zeros on both sides, so that the
-// shifted reads need no bounds checks.
+// shifted reads need no bounds checks.  An infinite or NaN entry of SF would make
+// NaN of the zeros, in entries of H that it has no part in, so those entries wait
+// until the others are summed (checks in the loop itself cost 8 to 57 % of the pass, this under 1 %).
 __global__ void __launch_bounds__(128) k_prod_conv(int B, int NJ, const double* __restrict__ d,
                                                    const double2* __restrict__ F, const double2* __restrict__ G,
                                                    double2* __restrict__ H) {
@@ -40,6 +75,7 @@ __global__ void __launch_bounds__(128) k_prod_conv(int B, int NJ, const double* 
   const double2* Gb = G + b * per;
   for (int e = threadIdx.x; e < D * SW; e += blockDim.x) sg[e] = make_double2(0.0, 0.0);
   __syncthreads();
+  bool bad = false;
   for (int e = threadIdx.x; e < D * D; e += blockDim.x) {   // e = m + D n, the order of d and F
     const int mi = e % D, ni = e / D, l0 = max(abs(mi - lmax), abs(ni - lmax));
     double2 a = make_double2(0.0, 0.0), c = a;
@@ -50,10 +86,11 @@ __global__ void __launch_bounds__(128) k_prod_conv(int B, int NJ, const double* 
       a.x = fma(w, u.x, a.x); a.y = fma(w, u.y, a.y);
       c.x = fma(w, v.x, c.x); c.y = fma(w, v.y, c.y);
     }
-    sf[mi * D + ni] = a;
+    bad |= !finite2(a);
+    sf[mi * D + ni] = finite2(a) ? a : make_double2(0.0, 0.0);
     sg[mi * SW + kProdR + ni] = c;
   }
-  __syncthreads();
+  bad = __syncthreads_or(bad);
   const int NR = (D + kProdR - 1) / kProdR;            // groups of R outputs per row
   double2* Hj = H + (b * NJ + j) * (long long)D * D;
   for (int it = threadIdx.x; it < D * NR; it += blockDim.x) {
@@ -89,6 +126,10 @@ __global__ void __launch_bounds__(128) k_prod_conv(int B, int NJ, const double* 
 #pragma unroll
     for (int r = 0; r < kProdR; ++r)
       if (n0 + r < D) Hj[mi + (long long)D * (n0 + r)] = acc[r];
+  }
+  if (bad) {
+    __syncthreads();
+    prod_conv_nonfinite(B, dj, Fb, sf, sg, Hj);
   }
 }
 
