@@ -113,6 +113,26 @@ void* hp_plan::ws_get(const char* name, size_t bytes, int* status) {
   return q;
 }
 
+void* hp_plan::ws_get_units(const char* name, size_t unit, long long want, long long least, long long* units,
+                            int* status) {
+  for (auto& kv : ws)
+    if (kv.first == name && kv.second.p && kv.second.cut && kv.second.bytes >= unit * (size_t)least) {
+      *units = std::min(want, (long long)(kv.second.bytes / unit));
+      return kv.second.p;
+    }
+  for (long long n = want;; n = std::max(least, n / 2)) {
+    *status = HP_OK;
+    void* q = ws_get(name, unit * (size_t)n, status);
+    if (q) {
+      for (auto& kv : ws)
+        if (kv.first == name) kv.second.cut = n < want;
+      *units = n;
+      return q;
+    }
+    if (n <= least) return nullptr;
+  }
+}
+
 ProfScope::ProfScope(hp_plan* plan, const char* name, cudaStream_t stream) : p(plan), s(stream) {
   ++p->launches;
   if (!p->prof_on) return;

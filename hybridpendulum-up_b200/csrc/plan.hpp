@@ -28,6 +28,7 @@ struct hp_state;
 struct Buf {
   void* p = nullptr;
   size_t bytes = 0;
+  bool cut = false;   // holds fewer units than were asked for, because more could not be had (ws_get_units)
 };
 
 // Per-kernel-family CUDA-event timing (opt-in) and a launch counter.
@@ -91,6 +92,11 @@ struct hp_plan {
   // workspace (grow-only), keyed by name
   std::vector<std::pair<std::string, Buf>> ws;
   void* ws_get(const char* name, size_t bytes, int* status);
+  // A workspace buffer of units of `unit` bytes that a caller works through in
+  // chunks: want of them, or, where the memory or the budget does not hold that,
+  // a half of it, a quarter and so on down to least (units: how many it got).  A
+  // buffer that was cut is kept: growing it again would fail and free it each time.
+  void* ws_get_units(const char* name, size_t unit, long long want, long long least, long long* units, int* status);
   void ws_release(const char* name);   // frees a workspace buffer (re-created on demand)
   // workspace buffers freed so far (grown or released): what holds addresses of
   // the workspace, a captured graph above all, is stale once this has moved

@@ -19,7 +19,9 @@
 #pragma once
 #include "row_groups.hpp"
 
-// G of one chunk of omega points: half of the 126 MB L2
+// G of one chunk of omega points: half of the 126 MB L2.  A chunk has at least 32
+// points (the lanes of k_synth_beta) where the memory allows it: more than this
+// for complex FP64 from B = 26 on, and all of the L2 at B = 32 (132 MB).
 constexpr long long kSynthG = 64LL << 20;
 
 template <int B, typename T, bool CPLX> struct Synth2Cfg {
@@ -268,8 +270,10 @@ int synth2_launch(hp_plan* p, const c2<T>* Fp, void* f, long long nx, cudaStream
   const long long per_w = (long long)NM * NB2 * NB2 * (long long)sizeof(C);
   long long nwc = std::max(32LL, kSynthG / per_w / 32 * 32);
   nwc = std::min(nwc, (nx + 31) / 32 * 32);
-  C* G = (C*)p->ws_get("tf.G", (size_t)per_w * nwc, &st);
+  long long units = 0;   // whole tiles of PA points
+  C* G = (C*)p->ws_get_units("tf.G", (size_t)per_w * PA, nwc / PA, 1, &units, &st);
   if (st) return st;
+  nwc = units * PA;
   constexpr size_t smem = (size_t)Cfg::bytes(NB, PA);
   HP_CUDA_TRY(cudaFuncSetAttribute(k_synth_ga<B, T, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   constexpr int NGRP = (NB2 + NB - 1) / NB;
