@@ -64,11 +64,17 @@ template <int B, typename T> struct RealSynthCfg {
     return want_nn ? bn : bp;
   }
   static constexpr int NN = pick(true), P = pick(false);
-  // The rule of the dispatch: tables and buffers fit, at least a fifth of the
-  // threads have an FFT, and the two passes of synth2.cuh were slower (24^3, us,
-  // this / two passes: B = 8 FP32 119 / 171, B = 16 FP32 1209 / 1518, B = 12 FP64
-  // 943 / 1251; the other way at B = 5 FP32, 90 / 50, and B = 6 FP64, 145 / 100).
-  static constexpr bool ok = NN > 0 && B >= (sizeof(T) == 4 ? 6 : 7) && 10 * NN * B * P >= NT && nrows < 65536;
+  // The rule of the dispatch: tables and buffers of two nodes or more fit, and the
+  // bandlimit is not one of the smallest; elsewhere the two passes of synth2.cuh
+  // are faster.  24^3, us, this / two passes: B = 8 FP32 119 / 171, B = 16 FP32
+  // 1209 / 1518, B = 12 FP64 943 / 1251; the other way at B = 5 FP32, 90 / 50, and
+  // B = 6 FP64, 145 / 100.  The upper edge, at 16^3: FP32 B = 16 379 / 418, B = 17
+  // 629 / 818; FP64 B = 16 681 / 802.  With one node per block every coefficient is
+  // read B times and a quarter of the threads have an FFT: FP32 B = 18 968 / 784,
+  // FP64 B = 17 1761 / 1244, B = 18 1892 / 1283 (24 x 24 points: FP32 B = 18 152 /
+  // 116, FP64 B = 17 265 / 174).  Below about a thousand omega points the two passes
+  // fill the chip better at B = 16 already (16 x 16, FP32: 41 / 32).
+  static constexpr bool ok = NN > 1 && B >= (sizeof(T) == 4 ? 6 : 7) && nrows < 65536;
 };
 
 // Row m of the G planes keeps its gamma index j at j ^ x(m), so that the rows
