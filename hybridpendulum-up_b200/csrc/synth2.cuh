@@ -240,24 +240,18 @@ __global__ void k_dsyn_table(RowLayout L, const T* __restrict__ wig, int DS, T* 
   out[t] = r < L.nrows && b < 2 * L.B ? (T)(2 * L.rows[r].x + 1) * wig[(size_t)b * L.nrows + r] : (T)0;
 }
 
+// gkey: the workspace buffer of G
 template <int B, typename T, bool CPLX>
-int synth2_launch(hp_plan* p, const c2<T>* Fp, void* f, long long nx, cudaStream_t s) {
+int synth2_launch(hp_plan* p, const c2<T>* Fp, void* f, long long nx, const char* gkey, cudaStream_t s) {
   using C = c2<T>;
   using Cfg = Synth2Cfg<B, T, CPLX>;
   if (tw_init() != 0) { hp_set_error("twiddle table upload failed"); return HP_ERR_CUDA; }
   constexpr int NB2 = 2 * B, NM = Cfg::NM, PA = Cfg::PA, NB = Cfg::NB, NPAIR = NM * (2 * B - 1), DS = (NB2 + 3) / 4 * 4;
   int st = HP_OK;
-  const char* key = CPLX ? "tf.pairs_c" : "tf.pairs_r";
-  bool have = false;
-  for (auto& kv : p->ws) if (kv.first == key) have = true;
-  int2* dpairs = (int2*)p->ws_get(key, sizeof(int2) * NPAIR, &st);
+  const int2* dpairs = pair_table<B, CPLX>(p, &st, s);
   if (st) return st;
-  if (!have) {
-    st = build_pairs<B, CPLX>(p, dpairs);
-    if (st) return st;
-  }
   const char* dkey = sizeof(T) == 8 ? "tf.dsyn64" : "tf.dsyn32";
-  have = false;
+  bool have = false;
   for (auto& kv : p->ws) if (kv.first == dkey) have = true;
   T* dtab = (T*)p->ws_get(dkey, sizeof(T) * (p->nrows + kRowPad) * DS, &st);
   if (st) return st;
@@ -271,7 +265,7 @@ int synth2_launch(hp_plan* p, const c2<T>* Fp, void* f, long long nx, cudaStream
   long long nwc = std::max(32LL, kSynthG / per_w / 32 * 32);
   nwc = std::min(nwc, (nx + 31) / 32 * 32);
   long long units = 0;   // whole tiles of PA points
-  C* G = (C*)p->ws_get_units("tf.G", (size_t)per_w * PA, nwc / PA, 1, &units, &st);
+  C* G = (C*)p->ws_get_units(gkey, (size_t)per_w * PA, nwc / PA, 1, &units, &st);
   if (st) return st;
   nwc = units * PA;
   constexpr size_t smem = (size_t)Cfg::bytes(NB, PA);

@@ -234,11 +234,11 @@ static int omega_fft_any(hp_plan* p, const c2<Tin>* in, c2<T>* out, bool inv, cu
   extern template int synth_launch<b, float, true>(hp_plan*, const float2*, void*, cudaStream_t);         \
   extern template int synth_launch<b, double, false>(hp_plan*, const double2*, void*, cudaStream_t);      \
   extern template int synth_launch<b, double, true>(hp_plan*, const double2*, void*, cudaStream_t);       \
-  extern template int anal2_launch<b, float, false>(hp_plan*, const void*, const double*, float2*, long long, cudaStream_t);  \
-  extern template int anal2_launch<b, float, true>(hp_plan*, const void*, const double*, float2*, long long, cudaStream_t);   \
-  extern template int anal2_launch<b, double, false>(hp_plan*, const void*, const double*, double2*, long long, cudaStream_t); \
-  extern template int anal2_launch<b, double, true>(hp_plan*, const void*, const double*, double2*, long long, cudaStream_t); \
-  extern template int synth2_launch<b, double, false>(hp_plan*, const double2*, void*, long long, cudaStream_t);
+  extern template int anal2_launch<b, float, false>(hp_plan*, const void*, const double*, float2*, long long, const char*, cudaStream_t);\
+  extern template int anal2_launch<b, float, true>(hp_plan*, const void*, const double*, float2*, long long, const char*, cudaStream_t);\
+  extern template int anal2_launch<b, double, false>(hp_plan*, const void*, const double*, double2*, long long, const char*, cudaStream_t);\
+  extern template int anal2_launch<b, double, true>(hp_plan*, const void*, const double*, double2*, long long, const char*, cudaStream_t);\
+  extern template int synth2_launch<b, double, false>(hp_plan*, const double2*, void*, long long, const char*, cudaStream_t);
 HP_FOR_EACH_B(X)
 #undef X
 
@@ -293,7 +293,7 @@ static int backward_T(hp_plan* p, const double2* Fint, void* f, int complex_out,
 template <typename T, bool CPLX>
 static int anal2_any(hp_plan* p, const void* f, const double* mult, c2<T>* out, cudaStream_t s) {
   switch (p->B) {
-#define X(b) case b: return anal2_launch<b, T, CPLX>(p, f, mult, out, p->nx, s);
+#define X(b) case b: return anal2_launch<b, T, CPLX>(p, f, mult, out, p->nx, "tf.Q", s);
     HP_FOR_EACH_B(X)
 #undef X
     default:
@@ -361,10 +361,11 @@ int hp_forward_internal_T(hp_plan* p, const void* f, const double* mult, void* o
 }
 
 // FP64 SO(3) transforms of nb real functions f (2B, 2B, 2B, nb) without omega
-// axes, HP_REAL plans of any precision: rows [row][nb].
+// axes, HP_REAL plans of any precision: rows [row][nb].  Their scratch is one
+// buffer of their own: the transforms of the plan's densities keep theirs, whatever nb.
 int hp_so3_forward64(hp_plan* p, const double* f, double2* rows, long long nb, cudaStream_t s) {
   switch (p->B) {
-#define X(b) case b: return anal2_launch<b, double, false>(p, f, nullptr, rows, nb, s);
+#define X(b) case b: return anal2_launch<b, double, false>(p, f, nullptr, rows, nb, "real.S", s);
     HP_FOR_EACH_B(X)
 #undef X
     default:
@@ -374,7 +375,7 @@ int hp_so3_forward64(hp_plan* p, const double* f, double2* rows, long long nb, c
 }
 int hp_so3_backward64(hp_plan* p, const double2* rows, double* f, long long nb, cudaStream_t s) {
   switch (p->B) {
-#define X(b) case b: return synth2_launch<b, double, false>(p, rows, f, nb, s);
+#define X(b) case b: return synth2_launch<b, double, false>(p, rows, f, nb, "real.S", s);
     HP_FOR_EACH_B(X)
 #undef X
     default:

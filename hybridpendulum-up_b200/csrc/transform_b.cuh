@@ -8,7 +8,6 @@
 // table, which the launchers fill before their first launch (tw_init).
 #pragma once
 #include <algorithm>
-#include <vector>
 #include "common.cuh"
 #include "plan.hpp"
 
@@ -62,30 +61,51 @@ __device__ __forceinline__ void stage_run(float* st, float* st2, const float2 (&
 }
 
 // (m, n) pairs with their row start, l-run length, m slot and n bin, longest
-// runs first (the order keeps the lanes of a warp on loops of similar length)
+// runs first (the order keeps the lanes of a warp on loops of similar length),
+// pairs of equal length by m, then n.  k = max(|m|, |n|) sets the length, so an
+// entry gives its pair in closed form: 4k + 1 pairs with m >= 0 have that k (two
+// for each m < k, 2k + 1 for m = k), 8k of all pairs (2k + 1 for m = -k, two for
+// each m between, 2k + 1 for m = k).  The device writes the table: a plan's first
+// transform waits for no copy from the host.
 template <int B, bool CPLX>
-static int build_pairs(hp_plan* p, int2* dpairs) {
-  constexpr int NB2 = 2 * B, NM = CPLX ? 2 * B - 1 : B, NPAIR = NM * (2 * B - 1);
-  std::vector<std::pair<int, int2>> v;
-  const int lmax = B - 1, D = 2 * lmax + 1, mlo = CPLX ? -lmax : 0;
-  for (int mi = 0; mi < NM; ++mi)
-    for (int n = -lmax; n <= lmax; ++n) {
-      const int m = mi + mlo;
-      const int lmin = std::max(std::abs(m), std::abs(n));
-      const int len = lmax - lmin + 1;
-      const int q = n >= 0 ? n : n + NB2;
-      int2 e;
-      e.x = p->h_seg[(size_t)(m - p->m_lo) * D + n + lmax];
-      e.y = len | (mi << 8) | (q << 16) | ((n == 0 ? 1 : 0) << 24);
-      v.push_back({len, e});
-    }
-  std::stable_sort(v.begin(), v.end(), [](const std::pair<int, int2>& a, const std::pair<int, int2>& b) {
-    return a.first > b.first;
-  });
-  std::vector<int2> h;
-  for (auto& x : v) h.push_back(x.second);
-  HP_CUDA_TRY(cudaMemcpy(dpairs, h.data(), sizeof(int2) * NPAIR, cudaMemcpyHostToDevice));
-  return HP_OK;
+__global__ void k_pairs(RowLayout L, int2* __restrict__ out) {
+  constexpr int lmax = B - 1, D = 2 * lmax + 1, NPAIR = (CPLX ? D : B) * D;
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= NPAIR) return;
+  auto first = [](int k) { return CPLX ? (k ? (2 * k - 1) * (2 * k - 1) : 0) : k * (2 * k - 1); };
+  int k = 0;
+  while (first(k + 1) <= q) ++k;
+  int r = q - first(k), m = k, n;
+  const int head = CPLX && k ? 2 * k + 1 : 0;          // the pairs with m = -k
+  const int mid = CPLX ? 2 * (2 * k - 1) : 2 * k;      // those between
+  if (k == 0) {
+    n = 0;
+  } else if (r < head) {
+    m = -k;
+    n = r - k;
+  } else if ((r -= head) < mid) {
+    m = (CPLX ? 1 - k : 0) + r / 2;
+    n = r & 1 ? k : -k;
+  } else {
+    n = r - mid - k;
+  }
+  const int mi = CPLX ? m + lmax : m, bin = n >= 0 ? n : n + 2 * B;
+  out[q] = make_int2(L.seg[(m - L.m_lo) * D + n + lmax], (B - k) | (mi << 8) | (bin << 16) | ((n == 0 ? 1 : 0) << 24));
+}
+
+// the plan's pair table
+template <int B, bool CPLX> static const int2* pair_table(hp_plan* p, int* st, cudaStream_t s) {
+  constexpr int NPAIR = (CPLX ? 2 * B - 1 : B) * (2 * B - 1);
+  const char* key = CPLX ? "tf.pairs_c" : "tf.pairs_r";
+  bool have = false;
+  for (auto& kv : p->ws) if (kv.first == key) have = true;
+  int2* t = (int2*)p->ws_get(key, sizeof(int2) * NPAIR, st);
+  if (*st) return nullptr;
+  if (!have) {
+    k_pairs<B, CPLX><<<(NPAIR + 127) / 128, 128, 0, s>>>(p->layout(), t);
+    if (cudaGetLastError() != cudaSuccess) { hp_set_error("pair table launch failed"); *st = HP_ERR_CUDA; }
+  }
+  return t;
 }
 
 // (2l+1) d^l_mn at the first B nodes as [group][row][NN], group g holding the
@@ -106,7 +126,7 @@ template <int B, typename T, bool CPLX>
 int synth_launch(hp_plan* p, const c2<T>* Fp, void* f, cudaStream_t s) {
   if (tw_init() != 0) { hp_set_error("twiddle table upload failed"); return HP_ERR_CUDA; }
   if constexpr (!CPLX && RealSynthCfg<B, T>::ok) return synth_real_launch<B, T>(p, Fp, reinterpret_cast<T*>(f), s);
-  else return synth2_launch<B, T, CPLX>(p, Fp, f, p->nx, s);
+  else return synth2_launch<B, T, CPLX>(p, Fp, f, p->nx, "tf.G", s);
 }
 
 // ----------------------------------------- analysis without atomics ----
@@ -367,8 +387,10 @@ __global__ void k_dw_table(RowLayout L, const T* __restrict__ wig, const double*
   dw[t] = (T)(qw[b] * (double)wig[(size_t)b * L.nrows + r]);
 }
 
+// qkey: the workspace buffer of Q
 template <int B, typename T, bool CPLX>
-int anal2_launch(hp_plan* p, const void* f, const double* mult, c2<T>* out, long long nx, cudaStream_t s) {
+int anal2_launch(hp_plan* p, const void* f, const double* mult, c2<T>* out, long long nx, const char* qkey,
+                 cudaStream_t s) {
   if (tw_init() != 0) { hp_set_error("twiddle table upload failed"); return HP_ERR_CUDA; }
   using C = c2<T>;
   using Cfg = AnalCfg<B, T, CPLX>;
@@ -378,17 +400,10 @@ int anal2_launch(hp_plan* p, const void* f, const double* mult, c2<T>* out, long
   int st = HP_OK;
   // pair table (shared with the synthesis) and the w_b d table
   constexpr int NPAIR = NM * (2 * B - 1);
-  const char* key = CPLX ? "tf.pairs_c" : "tf.pairs_r";
-  bool have = false;
-  for (auto& kv : p->ws) if (kv.first == key) have = true;
-  int2* dpairs = (int2*)p->ws_get(key, sizeof(int2) * NPAIR, &st);
+  const int2* dpairs = pair_table<B, CPLX>(p, &st, s);
   if (st) return st;
-  if (!have) {
-    st = build_pairs<B, CPLX>(p, dpairs);
-    if (st) return st;
-  }
   const char* dkey = sizeof(T) == 8 ? "tf.dw64" : "tf.dw32";
-  have = false;
+  bool have = false;
   for (auto& kv : p->ws) if (kv.first == dkey) have = true;
   T* dw = (T*)p->ws_get(dkey, sizeof(T) * p->nrows * NB2, &st);
   if (st) return st;
@@ -404,7 +419,7 @@ int anal2_launch(hp_plan* p, const void* f, const double* mult, c2<T>* out, long
   nwc = std::min(nwc, (nx + 31) / 32 * 32);
   RowLayout L = p->layout();
   L.nx = nx;
-  C* Qg = (C*)p->ws_get("tf.Q", (size_t)per_w * nwc, &st);
+  C* Qg = (C*)p->ws_get(qkey, (size_t)per_w * nwc, &st);
   if (st) return st;
   HP_CUDA_TRY(cudaFuncSetAttribute(k_anal_ag<B, T, PA, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   for (long long w0 = 0; w0 < nx; w0 += nwc) {
@@ -446,9 +461,9 @@ int anal2_launch(hp_plan* p, const void* f, const double* mult, c2<T>* out, long
   template int synth_launch<b, float, true>(hp_plan*, const float2*, void*, cudaStream_t);         \
   template int synth_launch<b, double, false>(hp_plan*, const double2*, void*, cudaStream_t);      \
   template int synth_launch<b, double, true>(hp_plan*, const double2*, void*, cudaStream_t);       \
-  template int anal2_launch<b, float, false>(hp_plan*, const void*, const double*, float2*, long long, cudaStream_t);  \
-  template int anal2_launch<b, float, true>(hp_plan*, const void*, const double*, float2*, long long, cudaStream_t);   \
-  template int anal2_launch<b, double, false>(hp_plan*, const void*, const double*, double2*, long long, cudaStream_t); \
-  template int anal2_launch<b, double, true>(hp_plan*, const void*, const double*, double2*, long long, cudaStream_t); \
-  template int synth2_launch<b, double, false>(hp_plan*, const double2*, void*, long long, cudaStream_t);
+  template int anal2_launch<b, float, false>(hp_plan*, const void*, const double*, float2*, long long, const char*, cudaStream_t);\
+  template int anal2_launch<b, float, true>(hp_plan*, const void*, const double*, float2*, long long, const char*, cudaStream_t);\
+  template int anal2_launch<b, double, false>(hp_plan*, const void*, const double*, double2*, long long, const char*, cudaStream_t);\
+  template int anal2_launch<b, double, true>(hp_plan*, const void*, const double*, double2*, long long, const char*, cudaStream_t);\
+  template int synth2_launch<b, double, false>(hp_plan*, const double2*, void*, long long, const char*, cudaStream_t);
 #endif
