@@ -322,7 +322,8 @@ int adjoint_apply(hp_plan* p, const double2* lam, const double2* F, double2* out
   int st = HP_OK;
   bool have = false;
   for (auto& kv : p->ws) if (kv.first == "adj.taps" && kv.second.p) have = true;
-  void* taps = p->ws_get("adj.taps", (p->precision == HP_FP64 ? sizeof(double) : sizeof(float)) * kTapStride * p->nrows, &st);
+  const size_t per = p->precision == HP_FP64 ? sizeof(double) * tap_stride<double>() : sizeof(float) * tap_stride<float>();
+  void* taps = p->ws_get("adj.taps", per * p->nrows, &st);
   if (st) return st;
   if (!have) ADJ_CHECK(hp_adjoint_gravity_taps(p, taps, s));
   q.taps = taps;

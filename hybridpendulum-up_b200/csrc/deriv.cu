@@ -86,57 +86,62 @@ __global__ void __launch_bounds__(128) k_axis3(RowLayout L, const c2<TIN>* __res
 // of the weights folds into nu[n2] = -i sum_i D_i gs_i MR_i^1_{0 n2}, so
 //   G = noise F + sum_{n2} nu[n2] sum_{l1} w(l1, n2) F^{l1}_{m, n-n2}.
 // Bound by the shared-memory pipe: 9 source values per output, and the row's
-// weights and sources, which come as whole vectors from tables built with the
+// weights and sources, which come as whole vectors from a table built with the
 // plan (one by one, with the sources recomputed by every block, the pass took
-// 0.49 ms at B = 15, 32^3, FP32 and 12.6 us at B = 8, 16 x 16; now 0.42 and 10.9).
+// 0.49 ms at B = 15, 32^3, FP32 and 12.6 us at B = 8, 16 x 16; now 0.42 and 8.8).
+// The sources are offsets in the padding of the weights' rows: as nine more
+// values of two bytes they took shared memory from the tile (FP64 B = 22, 64 x 64:
+// 371 us, 294 now, 342 before there was a table; B = 12, 24^3: 159 and 147).
 template <typename T> __host__ __device__ constexpr size_t local_tile_bytes(int rmax, int W) {
   return ((size_t)rmax * W * sizeof(c2<T>) + 15) / 16 * 16;
 }
 
-// The nine weights and nine sources of row r of an m group, read 16 bytes
-// (weights) and 8 bytes (sources) at a time.
+// The nine weights and the source offsets of one row of the tap tables, in whole
+// 16-byte reads.
 template <typename T> struct Taps {
-  T w[kTapStride];
-  short src[kTapStride];
-  __device__ __forceinline__ void load(const T* sw, const short* ssrc, int r) {
+  T w[tap_stride<T>()];
+  __device__ __forceinline__ void load(const T* row) {
     struct alignas(16) V { T v[16 / sizeof(T)]; };
 #pragma unroll
-    for (int k = 0; k < kTapStride; k += 16 / (int)sizeof(T))
-      *reinterpret_cast<V*>(w + k) = *reinterpret_cast<const V*>(sw + r * kTapStride + k);
-#pragma unroll
-    for (int k = 0; k < kTapStride; k += 4)
-      *reinterpret_cast<short4*>(src + k) = *reinterpret_cast<const short4*>(ssrc + r * kTapStride + k);
+    for (int k = 0; k < tap_stride<T>(); k += 16 / (int)sizeof(T))
+      *reinterpret_cast<V*>(w + k) = *reinterpret_cast<const V*>(row + k);
+  }
+  // tap t's source row less the row itself
+  __device__ __forceinline__ int off(int t) const {
+    if (t == 4) return 0;
+    const int k = t - (t > 4);
+    int word;
+    if constexpr (sizeof(T) == 8) word = k < 4 ? __double2loint(w[9]) : __double2hiint(w[9]);
+    else word = __float_as_int(k < 4 ? w[9] : w[10]);
+    return (word << (24 - 8 * (k & 3))) >> 24;
   }
 };
 
 template <typename T, int W, int NDIM, typename TIN>
 __global__ void __launch_bounds__(256) k_local(RowLayout L, const c2<TIN>* __restrict__ F,
                                                c2<T>* __restrict__ G, const T* __restrict__ tap_wr,
-                                               const short* __restrict__ tap_src, const c2<T>* __restrict__ Gx,
-                                               const c2<T>* __restrict__ sdk, DerivParams prm, int cpb) {
+                                               const c2<T>* __restrict__ Gx, const c2<T>* __restrict__ sdk,
+                                               DerivParams prm, int cpb) {
   using C = c2<T>;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int D = 2 * L.lmax + 1;
   const int rmax = (L.lmax + 1) * (L.lmax + 1);
   C* tile = reinterpret_cast<C*>(smraw);                                          // [R][W]
-  T* sw = reinterpret_cast<T*>(smraw + local_tile_bytes<T>(rmax, W));             // [R][kTapStride]
-  short* ssrc = reinterpret_cast<short*>(sw + (size_t)rmax * kTapStride);         // [R][kTapStride]
-  int* sseg = reinterpret_cast<int*>(ssrc + (size_t)rmax * kTapStride);           // [D]
+  constexpr int TS = tap_stride<T>();
+  T* sw = reinterpret_cast<T*>(smraw + local_tile_bytes<T>(rmax, W));             // [R][TS]
+  int* sseg = reinterpret_cast<int*>(sw + (size_t)rmax * TS);                     // [D]
   const int m = (int)blockIdx.y + L.m_lo;
   const int r0 = L.seg[(m - L.m_lo) * D];
   const int r1 = (m + 1 <= L.lmax) ? L.seg[(m + 1 - L.m_lo) * D] : (int)L.nrows;
   const int R = r1 - r0;
   const int tid = threadIdx.x, nth = blockDim.x;
-  // per block, once for its cpb omega chunks: the group's tap weights and tap
-  // sources, straight copies of the tables (the tap t = (l1 - l + 1) * 3 +
-  // (n2 + 1) of row r reads group row src[r][t], row 0 where it has no weight,
-  // so the tap loop below has no branches)
+  // per block, once for its cpb omega chunks: the group's rows of the tap table
+  // (a tap without weight reads the row itself, so the tap loop below has no
+  // branches)
   {
     constexpr int EP = 16 / (int)sizeof(T);
-    const T* tw = tap_wr + (size_t)r0 * kTapStride;
-    const short* ts = tap_src + (size_t)r0 * kTapStride;
-    for (int e = tid; e < R * kTapStride / EP; e += nth) cp_async<16>(sw + e * EP, tw + e * EP, true);
-    for (int e = tid; e < R * kTapStride / 4; e += nth) cp_async<8>(ssrc + e * 4, ts + e * 4, true);
+    const T* tw = tap_wr + (size_t)r0 * TS;
+    for (int e = tid; e < R * TS / EP; e += nth) cp_async<16>(sw + e * EP, tw + e * EP, true);
   }
   if (sdk)
     for (int e = tid; e < D; e += nth) sseg[e] = L.seg[(m - L.m_lo) * D + e] - r0;
@@ -213,14 +218,14 @@ __global__ void __launch_bounds__(256) k_local(RowLayout L, const c2<TIN>* __res
       const C f0 = tile[r * W + w];
       T ax = noise * f0.x, ay = noise * f0.y;
       Taps<T> tap;
-      tap.load(sw, ssrc, r);
+      tap.load(sw + r * TS);
 #pragma unroll
       for (int n2o = 0; n2o < 3; ++n2o) {
         T sx = 0, sy = 0;
 #pragma unroll
         for (int l1o = 0; l1o < 3; ++l1o) {
           const T wt = tap.w[l1o * 3 + n2o];
-          const C fs = tile[tap.src[l1o * 3 + n2o] * W + w];
+          const C fs = tile[(r + tap.off(l1o * 3 + n2o)) * W + w];
           sx = fma(wt, fs.x, sx);
           sy = fma(wt, fs.y, sy);
         }
@@ -257,8 +262,7 @@ __global__ void __launch_bounds__(256) k_local(RowLayout L, const c2<TIN>* __res
 
 template <typename T> static size_t local_smem(const hp_plan* p, int W) {
   const int rmax = (p->lmax + 1) * (p->lmax + 1);
-  return local_tile_bytes<T>(rmax, W) + (sizeof(T) + sizeof(short)) * (size_t)rmax * kTapStride +
-         sizeof(int) * ((p->D + 3) / 4 * 4);
+  return local_tile_bytes<T>(rmax, W) + sizeof(T) * (size_t)rmax * tap_stride<T>() + sizeof(int) * ((p->D + 3) / 4 * 4);
 }
 template <typename T> static const T* tap_table(const hp_plan* p);
 template <> const double* tap_table<double>(const hp_plan* p) { return p->tap_wr; }
@@ -266,8 +270,6 @@ template <> const float* tap_table<float>(const hp_plan* p) { return p->tap_wr32
 template <typename T> static const c2<T>* so3d_table(const hp_plan* p);
 template <> const double2* so3d_table<double>(const hp_plan* p) { return p->so3d64; }
 template <> const float2* so3d_table<float>(const hp_plan* p) { return p->so3d32; }
-
-template <typename T> static constexpr int local_w() { return sizeof(T) == 8 ? 16 : 32; }
 
 // --------------------------------------------------- pass C: plane pass ----
 
@@ -770,41 +772,49 @@ static int local_w_launch(hp_plan* p, const c2<TIN>* F, c2<T>* G, const c2<T>* G
   ProfScope _ps(p, "deriv.local", s);
   if (p->ndim == 3) {
     HP_CUDA_TRY(cudaFuncSetAttribute(k_local<T, W, 3, TIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsm));
-    k_local<T, W, 3, TIN><<<grid, 256, lsm, s>>>(p->layout(), F, G, taps, p->tap_src, Gx, so3d_table<T>(p), prm, cpb);
+    k_local<T, W, 3, TIN><<<grid, 256, lsm, s>>>(p->layout(), F, G, taps, Gx, so3d_table<T>(p), prm, cpb);
   } else {
     HP_CUDA_TRY(cudaFuncSetAttribute(k_local<T, W, 2, TIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsm));
-    k_local<T, W, 2, TIN><<<grid, 256, lsm, s>>>(p->layout(), F, G, taps, p->tap_src, Gx, so3d_table<T>(p), prm, cpb);
+    k_local<T, W, 2, TIN><<<grid, 256, lsm, s>>>(p->layout(), F, G, taps, Gx, so3d_table<T>(p), prm, cpb);
   }
   HP_CUDA_TRY(cudaGetLastError());
   return HP_OK;
 }
 
-// k_local with the widest omega tile (32/16/8/4 points) whose group tile and
-// tap weights fit 110 KB of shared memory (the m = 0 group has (lmax+1)^2 rows)
-// and that leaves enough blocks, or whose half would leave threads of the widest
-// group without a row: on small grids a block walks its rows in a serial chain
-// while SMs idle.  RK4 step with density, us, widest that fits / this: FP32 2-D
-// B = 8, 16^2 69.7 / 61.5, B = 12, 16^2 117 / 95, B = 16, 16^2 178 / 145; FP64
-// B = 16, 16^2 202 / 193.  The lines, us: 2-D, 16 points, 256 blocks (FP64 B = 16,
-// 16^2) 202 against 193 at 8, 288 (B = 8, 24^2) 86.5 against 88.6; 32 points (the
-// FP64 state is read: 16 are still 256 bytes), 288 blocks (FP32 B = 16, 24^2)
-// 331 against 298 at 16, 512 (32^2) 535 against 508.  3-D (three passes share the
-// step, FP32 input): 512 blocks of 32 (FP32 B = 4, 16^3) 88 against 98 at 16, 128
-// (B = 8, 8^3) 110.7 at 32 and 16, 111.8 at 8.  Half the threads idle at 8 points
-// for B = 4 (3-D, 8^3: 73.6 at 16, 77.5 at 8).
+// k_local with the widest omega tile (32/16/8/4 points) that leaves three blocks
+// per SM (72 KB of shared memory; the m = 0 group has (lmax+1)^2 rows) and enough
+// blocks on the chip, or whose half would leave threads of the widest group
+// without a row: on small grids a block walks its rows in a serial chain while
+// SMs idle.  FP64 keeps 8 points where two blocks fit (4 points are 64 bytes of a
+// row), FP32 where there are many blocks too (4 points are 32 bytes).
+// Two blocks at the wider tile against three at the narrower, us per pass: FP32
+// B = 16, 16^3 90 / 74 (32 and 16 points), B = 19, 48^2 146 / 123, B = 24, 24^2 84 /
+// 73 (16 and 8), 48^2 295 / 200; FP64 B = 18, 16^3 170 / 162; but 8 and 4 points: FP64
+// B = 22, 24^2 62 / 72, FP32 24^2 B = 30 165 / 124, 48^2 B = 28 (8064 blocks of 8 points)
+// 392 / 374, B = 31 (8928) 526 / 560, 60^2 B = 30 (13500) 730 / 761.
+// RK4 step with density, us, widest that fits / enough blocks: FP32 2-D B = 8, 16^2
+// 69.7 / 61.5, B = 12, 16^2 117 / 95; FP64 B = 16, 16^2 202 / 193.  The lines, us: 2-D, 16
+// points, 256 blocks (FP64 B = 16, 16^2) 202 against 193 at 8, 288 (B = 8, 24^2) 86.5
+// against 88.6; 32 points (the FP64 state is read: 16 are still 256 bytes), per
+// pass, 384 blocks (FP32 B = 12, 32^2) 18.9 against 16.8 at 16, 600 (40^2) 22.9
+// against 23.0, 864 (48^2) 27.0 against 31.2.  3-D (three passes share the step, FP32
+// input): 512 blocks of 32 (FP32 B = 4, 16^3) 88 against 98 at 16, 128 (B = 8, 8^3)
+// 110.7 at 32 and 16, 111.8 at 8.  Half the threads idle at 8 points for B = 4 (3-D,
+// 8^3: 73.6 at 16, 77.5 at 8).
 template <typename T, typename TIN = double>
 static int launch_local(hp_plan* p, const c2<TIN>* F, c2<T>* G, const c2<T>* Gx, const DerivParams& prm,
                         cudaStream_t s) {
-  constexpr size_t budget = 110 * 1024;
+  constexpr size_t three = 72 * 1024, two = 110 * 1024;   // shared memory for as many blocks per SM
   const int rmax = (p->lmax + 1) * (p->lmax + 1);
+  const auto blocks = [&](int W) { return (p->nx + W - 1) / W * p->nm; };
   const auto take = [&](int W) {
     const long long min_blocks = p->ndim == 3 ? 148 : W == 32 ? 592 : 280;
-    return local_smem<T>(p, W) <= budget &&
-           ((p->nx + W - 1) / W * p->nm >= min_blocks || rmax * (W / 2) < 256);
+    return local_smem<T>(p, W) <= three && (blocks(W) >= min_blocks || rmax * (W / 2) < 256);
   };
   if (sizeof(T) == 4 && take(32)) return local_w_launch<T, 32, TIN>(p, F, G, Gx, prm, s);
   if (take(16)) return local_w_launch<T, 16, TIN>(p, F, G, Gx, prm, s);
-  if (local_smem<T>(p, 8) <= budget) return local_w_launch<T, 8, TIN>(p, F, G, Gx, prm, s);
+  if (local_smem<T>(p, 8) <= (sizeof(T) == 8 || blocks(8) >= 8192 ? two : three))
+    return local_w_launch<T, 8, TIN>(p, F, G, Gx, prm, s);
   if (local_smem<T>(p, 4) <= (size_t)200 * 1024) return local_w_launch<T, 4, TIN>(p, F, G, Gx, prm, s);
   hp_set_error("gravity pass tiles exceed shared memory for this bandlimit");
   return HP_ERR_UNSUPPORTED;
@@ -1114,22 +1124,19 @@ int hp_derivative_eval_prm(hp_plan* p, const DerivParams& prm, const double2* Fe
 template <int W, int NDIM>
 __global__ void __launch_bounds__(256) k_local_dots(RowLayout L, const double2* __restrict__ F,
                                                     const double2* __restrict__ lam, const double* __restrict__ tap_wr,
-                                                    const short* __restrict__ tap_src, DerivParams prm, int cpb, int half, double scale,
+                                                    DerivParams prm, int cpb, int half, double scale,
                                                     double* __restrict__ acc, int nblocks, int slot) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int D = 2 * L.lmax + 1, rmax = (L.lmax + 1) * (L.lmax + 1);
   double2* tile = reinterpret_cast<double2*>(smraw);                                   // [R][W]
-  double* sw = reinterpret_cast<double*>(smraw + local_tile_bytes<double>(rmax, W));   // [R][kTapStride]
-  short* ssrc = reinterpret_cast<short*>(sw + (size_t)rmax * kTapStride);              // [R][kTapStride]
+  constexpr int TS = tap_stride<double>();
+  double* sw = reinterpret_cast<double*>(smraw + local_tile_bytes<double>(rmax, W));   // [R][TS]
   const int m = (int)blockIdx.y + L.m_lo;
   const int r0 = L.seg[(m - L.m_lo) * D];
   const int r1 = (m + 1 <= L.lmax) ? L.seg[(m + 1 - L.m_lo) * D] : (int)L.nrows;
   const int R = r1 - r0, N = L.N;
   const int tid = threadIdx.x, nth = blockDim.x;
-  for (int e = tid; e < R * kTapStride; e += nth) {
-    sw[e] = tap_wr[(size_t)r0 * kTapStride + e];
-    ssrc[e] = tap_src[(size_t)r0 * kTapStride + e];
-  }
+  for (int e = tid; e < R * TS; e += nth) sw[e] = tap_wr[(size_t)r0 * TS + e];
   const double tp = 2.0 * M_PI / prm.L, weight = scale * (half && m > 0 ? 2.0 : 1.0);
   const int w = tid % W, rl = tid / W, nrl = nth / W;
   const long long nchunks = (L.nx + W - 1) / W;
@@ -1153,15 +1160,17 @@ __global__ void __launch_bounds__(256) k_local_dots(RowLayout L, const double2* 
     for (int q = 0; q < 3; ++q) t[q] = make_double2(0.0, 0.0);
     for (int r = rl; r < R; r += nrl) {
       const double2 v = lam[(size_t)(r0 + r) * L.nx + wg], f0 = tile[r * W + w];
+      const double* tw = sw + r * TS;
+      const signed char* off = reinterpret_cast<const signed char*>(tw + 9);
       u += v.x * f0.x + v.y * f0.y;
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         double sx = 0.0, sy = 0.0;
 #pragma unroll
         for (int l1o = 0; l1o < 3; ++l1o) {
-          const int k = r * kTapStride + l1o * 3 + q;
-          const double wt = sw[k];
-          const double2 fs = tile[ssrc[k] * W + w];
+          const int k = l1o * 3 + q;
+          const double wt = tw[k];
+          const double2 fs = tile[(r + (k == 4 ? 0 : off[k - (k > 4)])) * W + w];
           sx = fma(wt, fs.x, sx);
           sy = fma(wt, fs.y, sy);
         }
@@ -1222,7 +1231,7 @@ static int local_dots_launch(hp_plan* p, const double2* F, const double2* lam, d
   ProfScope _ps(p, "adj.dot", s);
   auto launch = [&](auto kern) -> int {
     HP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsm));
-    kern<<<grid, 256, lsm, s>>>(p->layout(), F, lam, p->tap_wr, p->tap_src, prm, cpb, half, scale, acc, nblocks, slot);
+    kern<<<grid, 256, lsm, s>>>(p->layout(), F, lam, p->tap_wr, prm, cpb, half, scale, acc, nblocks, slot);
     HP_CUDA_TRY(cudaGetLastError());
     return HP_OK;
   };

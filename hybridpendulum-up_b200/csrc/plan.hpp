@@ -20,8 +20,11 @@ struct RowLayout {
   const int* seg;                   // first row of segment (m, n): seg[(m-m_lo)*(2lmax+1) + n+lmax]
 };
 
-// taps per row in the tables: nine, padded to whole 16-byte reads
-constexpr int kTapStride = 12;
+// Values per row in the gravity tap tables, whole 16-byte reads: the nine weights
+// and, in the eight bytes behind them, how far the source rows of the eight taps
+// other than the centre lie from the row itself (signed bytes; the row itself
+// where the tap has no weight).
+template <typename T> constexpr int tap_stride() { return sizeof(T) == 8 ? 10 : 12; }
 
 struct hp_state;
 
@@ -63,10 +66,9 @@ struct hp_plan {
   // model
   bool has_model = false;
   hp_model model{};
-  // [row][kTapStride] real gravity tap weights, tap (l1-l+1)*3 + (n2+1), zeros behind
+  // [row][tap_stride] real gravity tap weights, tap (l1-l+1)*3 + (n2+1), and source offsets
   double* tap_wr = nullptr;
   float* tap_wr32 = nullptr;
-  short* tap_src = nullptr;  // [row][kTapStride] the tap's row, counted from the first row of its m group
   double2 mr1[3][3] = {};    // MR_i^1_{0 n2} of the model: [n2+1][i]
   double* den_mR = nullptr;  // [2][(2B)^3] density-side gravity multipliers (pendulum_reduced_den)
   // attitude diffusion sum_ij G1_ij F^l u_i^T u_j^T of the gyro-bias model:
@@ -166,7 +168,7 @@ void hp_tune_apply_cached(hp_plan* p);
 int hp_tables_build(hp_plan* p);
 int hp_twiddles_init();
 int hp_build_gravity_taps(hp_plan* p);
-// the weights of W Grav W^-1, W = diag(2l+1), in the plan's compute precision (out: [row][kTapStride])
+// the weights of W Grav W^-1, W = diag(2l+1), in the plan's compute precision (out: [row][tap_stride])
 int hp_adjoint_gravity_taps(hp_plan* p, void* out, cudaStream_t s);
 int hp_full_to_internal(hp_plan* p, const double2* Ffull, double2* Fint, cudaStream_t s);
 // the same of the projection onto the real-density subspace, (F + C F) / 2

@@ -121,36 +121,33 @@ __global__ void k_cg1(int lmax, double* cg1) {
 // W = (2l1+1)*3/(2l+1) <l1 m; 1 0|l m><l1 n-n2; 1 n2|l n> MR_i^1_{0 n2}
 // (the l2 = 1, m2 = 0 terms of the CG loop of pendulum.m:474-502).  The
 // weight factors into a real part per tap, stored here as
-// tap_wr[row*kTapStride + (l1-l+1)*3 + (n2+1)] (zero where the source row does
-// not exist), and the model's MR_i^1_{0 n2}, applied per omega point.  tap_src
-// (may be null): the tap's source row within the row's m group, 0 for a tap
-// without weight.
+// tap_wr[row*tap_stride + (l1-l+1)*3 + (n2+1)] (zero where the source row does
+// not exist) with the offset of the source row behind (tap_stride), and the
+// model's MR_i^1_{0 n2}, applied per omega point.
 // ADJ: the weights of W Grav W^-1 with W = diag(2l+1), the adjoint's gravity.
 template <typename T, bool ADJ = false>
-__global__ void k_gravity_taps(RowLayout L, const double* __restrict__ cg1, T* __restrict__ tap_wr,
-                               short* __restrict__ tap_src) {
+__global__ void k_gravity_taps(RowLayout L, const double* __restrict__ cg1, T* __restrict__ tap_wr) {
   const long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (r >= L.nrows) return;
   const int lmax = L.lmax;
   const char4 q = L.rows[r];
   const int l = q.x, m = q.y, n = q.z;
+  T* wr = tap_wr + r * tap_stride<T>();
+  for (int t = 9; t < tap_stride<T>(); ++t) wr[t] = (T)0;
+  signed char* off = reinterpret_cast<signed char*>(wr + 9);
   for (int t = 0; t < 9; ++t) {
     const int l1 = l + t / 3 - 1, n2 = t % 3 - 1, n1 = n - n2;
     double w = 0.0;
-    int src = 0;
+    long long src = r;
     if (l1 >= 0 && l1 <= lmax && abs(m) <= l1 && abs(n1) <= l1) {
-      const int D = 2 * lmax + 1, g = (m - L.m_lo) * D;
-      src = L.seg[g + n1 + lmax] - L.seg[g] + l1 - max(abs(m), abs(n1));
+      // rows of adjacent n are at most B + 2 apart
+      src = L.seg[(m - L.m_lo) * (2 * lmax + 1) + n1 + lmax] + l1 - max(abs(m), abs(n1));
       const double cm = cg1[cg1_index(lmax, l1, l - l1, m, 0)];
       const double cn = cg1[cg1_index(lmax, l1, l - l1, n, n2)];
       w = ADJ ? 3.0 * cm * cn : (2.0 * l1 + 1.0) * 3.0 / (2.0 * l + 1.0) * cm * cn;
     }
-    tap_wr[r * kTapStride + t] = (T)w;
-    if (tap_src) tap_src[r * kTapStride + t] = (short)src;
-  }
-  for (int t = 9; t < kTapStride; ++t) {
-    tap_wr[r * kTapStride + t] = (T)0;
-    if (tap_src) tap_src[r * kTapStride + t] = 0;
+    wr[t] = (T)w;
+    if (t != 4) off[t - (t > 4)] = (signed char)(src - r);
   }
 }
 
@@ -406,25 +403,23 @@ int hp_tables_on_grid(hp_plan* p, int Bg, double* fact, double* d, double* w, cu
 
 int hp_build_gravity_taps(hp_plan* p) {
   if (p->tap_wr) return HP_OK;
-  // weights in both precisions and the sources in one buffer (each part a
-  // multiple of 8 bytes per row)
+  // both precisions in one buffer (rows of 80 and 48 bytes)
   char* buf = nullptr;
-  const size_t n = (size_t)kTapStride * p->nrows;
-  HP_CUDA_TRY(hp_dev_alloc(&buf, (sizeof(double) + sizeof(float) + sizeof(short)) * n));
+  const size_t n = (size_t)p->nrows;
+  HP_CUDA_TRY(hp_dev_alloc(&buf, (sizeof(double) * tap_stride<double>() + sizeof(float) * tap_stride<float>()) * n));
   p->tap_wr = reinterpret_cast<double*>(buf);
-  p->tap_wr32 = reinterpret_cast<float*>(p->tap_wr + n);
-  p->tap_src = reinterpret_cast<short*>(p->tap_wr32 + n);
+  p->tap_wr32 = reinterpret_cast<float*>(p->tap_wr + tap_stride<double>() * n);
   const unsigned g = (unsigned)((p->nrows + 127) / 128);
-  k_gravity_taps<double><<<g, 128, 0, p->stream>>>(p->layout(), p->cg1, p->tap_wr, p->tap_src);
-  k_gravity_taps<float><<<g, 128, 0, p->stream>>>(p->layout(), p->cg1, p->tap_wr32, nullptr);
+  k_gravity_taps<double><<<g, 128, 0, p->stream>>>(p->layout(), p->cg1, p->tap_wr);
+  k_gravity_taps<float><<<g, 128, 0, p->stream>>>(p->layout(), p->cg1, p->tap_wr32);
   HP_CUDA_TRY(cudaGetLastError());
   return HP_OK;
 }
 
 int hp_adjoint_gravity_taps(hp_plan* p, void* out, cudaStream_t s) {
   const unsigned g = (unsigned)((p->nrows + 127) / 128);
-  if (p->precision == HP_FP64) k_gravity_taps<double, true><<<g, 128, 0, s>>>(p->layout(), p->cg1, (double*)out, nullptr);
-  else k_gravity_taps<float, true><<<g, 128, 0, s>>>(p->layout(), p->cg1, (float*)out, nullptr);
+  if (p->precision == HP_FP64) k_gravity_taps<double, true><<<g, 128, 0, s>>>(p->layout(), p->cg1, (double*)out);
+  else k_gravity_taps<float, true><<<g, 128, 0, s>>>(p->layout(), p->cg1, (float*)out);
   HP_CUDA_TRY(cudaGetLastError());
   return HP_OK;
 }
