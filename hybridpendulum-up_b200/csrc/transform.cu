@@ -29,11 +29,12 @@ using namespace hp;
 // nrows * P values.  B = 15, 24^3, FP32: synthesis 1025 -> 882 us for 20 us more
 // in the plane pass's stores.
 
-// Distance of two planes in shared memory: N rows of N + 1 values, padded so
-// that the rows' pieces of one omega block (4 FP32 or 2 FP64 points each) sit
-// on distinct banks when the blocked store reads them one after another
+// Distance of two planes in shared memory: N rows of N + 1 values, for the blocked
+// store padded so that the rows' pieces of one omega block (4 FP32 or 2 FP64
+// points each) sit on distinct banks when it reads them one after another
 // (B = 15, 32^3, FP32: 0.29 -> 0.2 ms).
-template <int N, typename T> __host__ __device__ constexpr int wplane_ps() {
+template <int N, typename T, bool BLK> __host__ __device__ constexpr int wplane_ps() {
+  if (!BLK) return N * (N + 1);
   constexpr int U = sizeof(T) == 4 ? 16 : 8, r = (N * (N + 1)) % U;   // values per 128-byte wavefront
   return N * (N + 1) + (U / 4 - r + U) % U;
 }
@@ -42,41 +43,44 @@ template <int N, typename T> __host__ __device__ constexpr int wplane_ps() {
 // plane give the 128 threads one FFT each, within 64 KB of shared memory.
 template <int N, typename T> __host__ __device__ constexpr int wplane_ppb() {
   constexpr int want = 128 / N > 1 ? 128 / N : 1;
-  constexpr int fit = (int)((64 * 1024) / ((size_t)wplane_ps<N, T>() * sizeof(c2<T>)));
+  constexpr int fit = (int)((64 * 1024) / ((size_t)wplane_ps<N, T, true>() * sizeof(c2<T>)));
   return want < fit ? want : (fit > 1 ? fit : 1);
 }
 
 // 2-D FFT over (k1, k2) of every (row, k3) plane; PPB consecutive planes (one
 // contiguous run of PPB N^2 values) per block.
-// blk > 0: the output goes to the omega-blocked layout of the synthesis input
+// BLK: the output goes to the omega-blocked layout of the synthesis input
 // (above); the block's planes are then the same k3 plane of PPB
 // consecutive rows, whose blk-point pieces are neighbours in that layout.  in
-// may equal out for blk = 0 (a block reads all of its planes before it writes).
-template <int N, typename Tin, typename T, bool INV>
+// may equal out otherwise (a block reads all of its planes before it writes).
+// Two kernels: with blk a run-time switch the contiguous one paid for the other's
+// index arithmetic (FP64, B = 22, 64 x 64, four transforms: 1175 -> 1240 us).
+template <int N, typename Tin, typename T, bool INV, bool BLK>
 __global__ void __launch_bounds__(128) k_wplane(const c2<Tin>* __restrict__ in, c2<T>* __restrict__ out,
-                                                long long nplanes, T scale, int blk = 0, long long nrows = 0,
-                                                int planes_per_row = 1) {
+                                                long long nplanes, T scale, int blk, long long nrows,
+                                                int planes_per_row) {
   using C = c2<T>;
   constexpr int PPB = wplane_ppb<N, T>();
-  constexpr int PS = wplane_ps<N, T>();
+  constexpr int PS = wplane_ps<N, T, BLK>();
   extern __shared__ __align__(16) unsigned char smraw[];
   C* sm = reinterpret_cast<C*>(smraw);   // [PPB][N][N+1], planes PS apart
   // planes of the block: consecutive ones, PS0 = N^2 values apart in memory;
   // for blocked output the same plane of consecutive rows, so that every omega
   // block of the output gets one contiguous run of np * blk values
   const long long rgroups = (nrows + PPB - 1) / PPB;
-  const long long pl0 = blk > 0 ? (long long)(blockIdx.x % rgroups) * PPB * planes_per_row + blockIdx.x / rgroups
-                                : (long long)blockIdx.x * PPB;
-  const long long PS0 = blk > 0 ? (long long)N * N * planes_per_row : (long long)N * N;
+  const long long pl0 = BLK ? (long long)(blockIdx.x % rgroups) * PPB * planes_per_row + blockIdx.x / rgroups
+                            : (long long)blockIdx.x * PPB;
+  const long long PS0 = (long long)N * N * planes_per_row;
   if (pl0 >= nplanes) return;
-  const int np = (int)min((long long)PPB, blk > 0 ? nrows - pl0 / planes_per_row : nplanes - pl0);
+  const int np = (int)min((long long)PPB, BLK ? nrows - pl0 / planes_per_row : nplanes - pl0);
   const int tot = np * N * N;
   const c2<Tin>* src = in + pl0 * N * N;
+  auto at = [&](int e) -> const c2<Tin>* { return BLK ? src + (e / (N * N)) * PS0 + e % (N * N) : src + e; };
   if constexpr (sizeof(Tin) == sizeof(T)) {
     // no conversion: the block's whole run is in flight at once (cp.async,
     // no register round trip)
     for (int e = threadIdx.x; e < tot; e += blockDim.x)
-      cp_async<sizeof(C)>(sm + (e / (N * N)) * PS + ((e / N) % N) * (N + 1) + e % N, src + (e / (N * N)) * PS0 + e % (N * N), true);
+      cp_async<sizeof(C)>(sm + (e / (N * N)) * PS + ((e / N) % N) * (N + 1) + e % N, at(e), true);
     cp_async_wait_all();
   } else {
     for (int e0 = threadIdx.x; e0 < tot; e0 += 4 * blockDim.x) {
@@ -84,7 +88,7 @@ __global__ void __launch_bounds__(128) k_wplane(const c2<Tin>* __restrict__ in, 
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int e = e0 + u * blockDim.x;
-        v[u] = e < tot ? cvt<C, c2<Tin>>(src[(e / (N * N)) * PS0 + e % (N * N)]) : czero<C>();
+        v[u] = e < tot ? cvt<C, c2<Tin>>(*at(e)) : czero<C>();
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -114,7 +118,7 @@ __global__ void __launch_bounds__(128) k_wplane(const c2<Tin>* __restrict__ in, 
     for (int j = 0; j < N; ++j) col[j * (N + 1)] = scale * x[j];
   }
   __syncthreads();
-  if (blk > 0) {
+  if constexpr (BLK) {
     const long long row0 = pl0 / planes_per_row, w0 = (pl0 % planes_per_row) * (long long)(N * N);
     // blocks do not straddle planes: consecutive threads write consecutive
     // values (row, w % blk) of one block
@@ -186,19 +190,18 @@ static int omega_fft(hp_plan* p, const c2<Tin>* in, c2<T>* out, bool inv, cudaSt
   const int ppr = p->ndim == 3 ? N : 1;
   const long long nplanes = p->nrows * ppr;
   constexpr int PPB = wplane_ppb<N, T>();
-  const size_t smem = sizeof(c2<T>) * PPB * wplane_ps<N, T>();
+  const size_t smem = sizeof(c2<T>) * PPB * (blk > 0 ? wplane_ps<N, T, true>() : wplane_ps<N, T, false>());
   const unsigned nblk = (unsigned)(blk > 0 ? (p->nrows + PPB - 1) / PPB * ppr : (nplanes + PPB - 1) / PPB);
   auto plane = [&](T sc) -> int {
     ProfScope _ps(p, "tf.wplane", s);
-    if (inv) {
-      HP_CUDA_TRY(cudaFuncSetAttribute(k_wplane<N, Tin, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_wplane<N, Tin, T, true><<<nblk, 128, smem, s>>>(in, out, nplanes, sc, blk, p->nrows, ppr);
-    } else {
-      HP_CUDA_TRY(cudaFuncSetAttribute(k_wplane<N, Tin, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_wplane<N, Tin, T, false><<<nblk, 128, smem, s>>>(in, out, nplanes, sc, blk, p->nrows, ppr);
-    }
-    HP_CUDA_TRY(cudaGetLastError());
-    return HP_OK;
+    auto go = [&](auto kern) -> int {
+      HP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      kern<<<nblk, 128, smem, s>>>(in, out, nplanes, sc, blk, p->nrows, ppr);
+      HP_CUDA_TRY(cudaGetLastError());
+      return HP_OK;
+    };
+    if (!inv) return go(k_wplane<N, Tin, T, false, false>);
+    return blk > 0 ? go(k_wplane<N, Tin, T, true, true>) : go(k_wplane<N, Tin, T, true, false>);
   };
   if (p->ndim == 3) {
     // plane pass (k1,k2) then line pass along k3, scale applied in the line pass
