@@ -24,8 +24,9 @@
 // fftSO3_prod.m:103-120 (two entries per row), so the transforms run on the
 // FFT kernels of the omega-batched transforms, the functions in the place of
 // omega points, and one pass changes the basis.  B = 16, 64 functions, forward
-// and backward: the direct sums 0.54 ms, this route 0.10 ms.  Complex plans hold
-// no tables for real functions and keep the direct sums.
+// and backward: the direct sums 0.54 ms, this route 0.10 ms.  Small batches of
+// small bandlimits keep the direct sums, two kernels for three (use_rows); so do
+// complex plans, which hold no tables for real functions.
 #include <cmath>
 #include <vector>
 #include "common.cuh"
@@ -219,6 +220,21 @@ static const double* real_psi(hp_plan* p, int* st) {
   return psi;
 }
 
+// The route of nb functions.  The direct sums are O(B^4) per function, the rows
+// O(B^3 log B) but one more launch: below B = 9 the sums are faster up to a batch
+// that falls as B^-2.  Whole call, us, sums / rows: forward B = 2, 500 functions
+// 25.2 / 24.5, 200 20.8 / 24.5; B = 5, 64 26.0 / 28.5, 100 28.9 / 28.7; B = 7, 32 29.9 /
+// 30.4, 48 33.4 / 30.1; B = 8, 12 30.0 / 30.3, 20 31.9 / 30.4; B = 9, 1 31.2 / 29.8.
+// Backward (its sums are the cheaper ones) B = 2, 500 23.2 / 27.1, 1000 27.5 / 27.0;
+// B = 5, 140 27.1 / 29.1, 200 30.8 / 29.6; B = 6, 64 26.4 / 28.7, 128 32.6 / 28.8; B = 8,
+// 24 26.7 / 28.0, 32 28.3 / 29.5; B = 9, 4 26.1 / 25.4.
+static bool use_rows(const hp_plan* p, int nb, bool forward) {
+  if (p->symmetry != HP_REAL) return false;
+  const int B = p->B;
+  const long long line = forward ? (B < 8 ? 1800 : 1024) : (B < 6 ? 4000 : 2600);
+  return B > 8 || (long long)nb * B * B > line;
+}
+
 static int real_args(hp_plan* p, const void* a, const void* b, int nbatch, int mem) {
   if (!p || !a || !b) { hp_set_error("null argument"); return HP_ERR_INVALID; }
   if (mem != HP_DEVICE && mem != HP_HOST) { hp_set_error("mem must be HP_DEVICE or HP_HOST"); return HP_ERR_INVALID; }
@@ -241,7 +257,7 @@ extern "C" int hp_fftSO3_real_forward(hp_plan* p, const double* f, double* F, in
     HP_CUDA_TRY(cudaMemcpyAsync(a, f, sizeof(double) * nf, cudaMemcpyHostToDevice, p->stream));
     fd = a;
   }
-  if (p->symmetry == HP_REAL) {
+  if (use_rows(p, nbatch, true)) {
     HP_CHECK(real_forward_rows(p, fd, Fd, nbatch, p->stream));
   } else {
     const double* psi = real_psi(p, &st);
@@ -276,7 +292,7 @@ extern "C" int hp_fftSO3_real_backward(hp_plan* p, const double* F, double* f, i
     HP_CUDA_TRY(cudaMemcpyAsync(a, F, sizeof(double) * nF, cudaMemcpyHostToDevice, p->stream));
     Fd = a;
   }
-  if (p->symmetry == HP_REAL) {
+  if (use_rows(p, nbatch, false)) {
     HP_CHECK(real_backward_rows(p, Fd, fd, nbatch, p->stream));
   } else {
     const double* psi = real_psi(p, &st);
