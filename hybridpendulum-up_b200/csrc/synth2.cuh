@@ -6,7 +6,8 @@
 //                 coefficients stays in registers, every beta's sum
 //                 G_b[m][n] = sum_l (2l+1) d^l_mn(beta_b) F^l_mn goes to G;
 //   k_synth_ga    block = NB betas x PA omega points: gamma FFT over n, alpha
-//                 FFT over m, the 2B-runs of the density leave by bulk copies.
+//                 FFT over m, the 2B-runs of the density leave by bulk copies;
+//                 on small grids it forms the sums itself (synth_fused).
 // What bounds it: G is written and read once (NM * 2B values per omega point
 // and beta).  The omega points are taken in chunks whose G stays in L2, so that
 // HBM sees little more than F and the density.  The one-kernel form before read
@@ -48,9 +49,23 @@ template <int B, typename T, bool CPLX> struct Synth2Cfg {
     return nb;
   }
   static constexpr int NB = pick_nb();
+  static constexpr bool fusable = B <= 6;   // see synth_fused
   // blocks per SM the registers allow
   static constexpr int MINB = NT == 256 ? 1 : sizeof(T) == 8 ? 2 : (NB2 <= 24 ? 5 : NB2 <= 40 ? 4 : 2);
 };
+
+// Small grids of small bandlimits take one kernel, k_synth_ga forming its own sums:
+// there the second launch costs more than reading the coefficients once per
+// group of betas.  Density call, us, one kernel before there were two / two / this:
+// real FP32 B = 3, 8 x 8 10.4 / 12.4 / 8.4, B = 5, 24 x 24 15.9 / 16.5 / 14.5; complex
+// FP32 B = 5, 24 x 24 16.5 / 18.6 / 16.5; real FP64 B = 4, 4^3 13.4 / 15.4 / 13.4.  The
+// lines: FP64 B = 5, 24 x 24 (72000) 16.6 either way, B = 4, 16^3 (262144) 23.7 two,
+// 27.8 one; FP32 real B = 4, 16^3 22.3 two, 18.6 one, complex B = 5, 12^3 (216000) 24.7
+// either way, B = 5, 16^3 (512000) 35.0 two, 37.1 one.  B = 7 FP32 complex, 8 x 8: 12.5
+// two, 14.5 one.
+template <typename T> bool synth_fused(int B, long long nx) {
+  return B <= 6 && (long long)B * B * B * nx <= (sizeof(T) == 8 ? 64LL << 10 : 256LL << 10);
+}
 
 // dtab: [row][DS] (2l+1) d^l_mn(beta_b), DS = 2B rounded up to 4; Fp: [row][nx];
 // G: [w / PA][b][m][n bin ^ x(m)][w % PA] of the chunk's omega points.
@@ -112,9 +127,11 @@ __global__ void __launch_bounds__(128) k_synth_beta(long long nx, const c2<T>* _
   }
 }
 
-template <int B, typename T, bool CPLX>
+// FUSED: the tile of G is summed here, from Fp and the table (w0 = 0, G unused).
+template <int B, typename T, bool CPLX, bool FUSED>
 __global__ void __launch_bounds__(Synth2Cfg<B, T, CPLX>::NT, Synth2Cfg<B, T, CPLX>::MINB)
-    k_synth_ga(const c2<T>* __restrict__ G, void* __restrict__ fout, long long w0, long long nx) {
+    k_synth_ga(const c2<T>* __restrict__ G, void* __restrict__ fout, long long w0, long long nx,
+               const c2<T>* __restrict__ Fp, const T* __restrict__ dtab, const int2* __restrict__ pairs) {
   using C = c2<T>;
   using Cfg = Synth2Cfg<B, T, CPLX>;
   constexpr int NB2 = 2 * B, NM = Cfg::NM, NCOL = Cfg::NCOL, PA = Cfg::PA, NB = Cfg::NB, NT = Cfg::NT;
@@ -126,7 +143,32 @@ __global__ void __launch_bounds__(Synth2Cfg<B, T, CPLX>::NT, Synth2Cfg<B, T, CPL
   const int b0 = (blockIdx.x % NGRP) * NB, nbv = min(NB, NB2 - b0);
   const long long wb = blockIdx.x / NGRP;
   const int tid = threadIdx.x;
-  {
+  if constexpr (FUSED) {
+    constexpr int NPAIR = NM * (2 * B - 1), DS = (NB2 + 3) / 4 * 4;
+    for (int it = tid; it < NPAIR * PA; it += NT) {
+      const int2 pe = pairs[it / PA];
+      const int s = pe.x, len = pe.y & 0xff, mi = (pe.y >> 8) & 0xff, q = (pe.y >> 16) & 0xff, pt = it % PA;
+      const bool ok = wb * PA + pt < nx;
+      const C* src = Fp + (size_t)s * nx + (ok ? wb * PA + pt : 0);
+      const T* d = dtab + (size_t)s * DS + b0;       // a last group's unused betas read on, into the rows behind
+      C acc[NB];
+#pragma unroll
+      for (int u = 0; u < NB; ++u) acc[u] = czero<C>();
+#pragma unroll 4
+      for (int j = 0; j < len; ++j) {
+        const C v = src[(size_t)j * nx];
+#pragma unroll
+        for (int u = 0; u < NB; ++u) {
+          acc[u].x = fma(d[j * DS + u], v.x, acc[u].x);
+          acc[u].y = fma(d[j * DS + u], v.y, acc[u].y);
+        }
+      }
+      C* g = sG + (mi * NB2 + (q ^ Swz::x(mi))) * PA + pt;
+#pragma unroll
+      for (int u = 0; u < NB; ++u)
+        if (u < nbv) g[u * NM * NB2 * PA] = acc[u];
+    }
+  } else {
     const C* src = G + (wb * NB2 + b0) * NM * NB2 * PA;
     constexpr int EPP = 16 / (int)sizeof(C);
     const int n = nbv * NM * NB2 * PA / EPP;
@@ -261,6 +303,18 @@ int synth2_launch(hp_plan* p, const c2<T>* Fp, void* f, long long nx, const char
         p->layout(), sizeof(T) == 8 ? (const T*)(const void*)p->wig64 : (const T*)(const void*)p->wig32, DS, dtab);
     HP_CUDA_TRY(cudaGetLastError());
   }
+  constexpr size_t smem = (size_t)Cfg::bytes(NB, PA);
+  constexpr int NGRP = (NB2 + NB - 1) / NB;
+  if constexpr (Cfg::fusable) {
+    if (synth_fused<T>(B, nx)) {
+      HP_CUDA_TRY(cudaFuncSetAttribute(k_synth_ga<B, T, CPLX, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      ProfScope _ps(p, "tf.synth", s);
+      k_synth_ga<B, T, CPLX, true><<<(unsigned)((nx + PA - 1) / PA * NGRP), Cfg::NT, smem, s>>>(nullptr, f, 0, nx, Fp, dtab,
+                                                                                               dpairs);
+      HP_CUDA_TRY(cudaGetLastError());
+      return HP_OK;
+    }
+  }
   const long long per_w = (long long)NM * NB2 * NB2 * (long long)sizeof(C);
   long long nwc = std::max(32LL, kSynthG / per_w / 32 * 32);
   nwc = std::min(nwc, (nx + 31) / 32 * 32);
@@ -268,9 +322,7 @@ int synth2_launch(hp_plan* p, const c2<T>* Fp, void* f, long long nx, const char
   C* G = (C*)p->ws_get_units(gkey, (size_t)per_w * PA, nwc / PA, 1, &units, &st);
   if (st) return st;
   nwc = units * PA;
-  constexpr size_t smem = (size_t)Cfg::bytes(NB, PA);
-  HP_CUDA_TRY(cudaFuncSetAttribute(k_synth_ga<B, T, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  constexpr int NGRP = (NB2 + NB - 1) / NB;
+  HP_CUDA_TRY(cudaFuncSetAttribute(k_synth_ga<B, T, CPLX, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   for (long long w0 = 0; w0 < nx; w0 += nwc) {
     const long long nw = std::min(nwc, nx - w0);
     {
@@ -282,7 +334,7 @@ int synth2_launch(hp_plan* p, const c2<T>* Fp, void* f, long long nx, const char
       HP_CUDA_TRY(cudaGetLastError());
     }
     ProfScope _ps(p, "tf.synth", s);
-    k_synth_ga<B, T, CPLX><<<(unsigned)((nw + PA - 1) / PA * NGRP), Cfg::NT, smem, s>>>(G, f, w0, nx);
+    k_synth_ga<B, T, CPLX, false><<<(unsigned)((nw + PA - 1) / PA * NGRP), Cfg::NT, smem, s>>>(G, f, w0, nx, Fp, dtab, dpairs);
     HP_CUDA_TRY(cudaGetLastError());
   }
   return HP_OK;
