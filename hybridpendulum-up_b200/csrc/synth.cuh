@@ -68,12 +68,11 @@ template <int B, typename T> struct RealSynthCfg {
   // bandlimit is not one of the smallest; elsewhere the two passes of synth2.cuh
   // are faster.  24^3, us, this / two passes: B = 8 FP32 119 / 171, B = 16 FP32
   // 1209 / 1518, B = 12 FP64 943 / 1251; the other way at B = 5 FP32, 90 / 50, and
-  // B = 6 FP64, 145 / 100.  The upper edge, at 16^3: FP32 B = 16 379 / 418, B = 17
-  // 629 / 818; FP64 B = 16 681 / 802.  With one node per block every coefficient is
+  // B = 6 FP64, 145 / 100.  The upper edge, at 16^3: FP32 B = 16 359 / 418, B = 17
+  // 610 / 818; FP64 B = 16 662 / 802.  With one node per block every coefficient is
   // read B times and a quarter of the threads have an FFT: FP32 B = 18 968 / 784,
   // FP64 B = 17 1761 / 1244, B = 18 1892 / 1283 (24 x 24 points: FP32 B = 18 152 /
-  // 116, FP64 B = 17 265 / 174).  Below about a thousand omega points the two passes
-  // fill the chip better at B = 16 already (16 x 16, FP32: 41 / 32).
+  // 116, FP64 B = 17 265 / 174).  On 16 x 16 points they are level at B = 16 (FP32 33 / 32).
   static constexpr bool ok = NN > 1 && B >= (sizeof(T) == 4 ? 6 : 7) && nrows < 65536;
 };
 
@@ -110,10 +109,15 @@ __global__ void __launch_bounds__(RealSynthCfg<B, T>::NT, 1)
   const int grp = blockIdx.x % NG;
   const long long chunk = blockIdx.x / NG;
   const int b0 = grp * NN, cnt = min(NN, B - b0);
+  // tables by asynchronous copies, which land with those of the first batch.  By
+  // loads, round after round, they were a good part of a block's life on small
+  // grids (us, before / now: B = 9, 8 x 8 points, whole call 15.5 / 13.5; synthesis
+  // at B = 16, 16 x 16 41.4 / 33.3, 8^3 72 / 56, 16^3 379 / 359; FP64 16^3 681 / 663)
   {
-    const T* src = dtab + (size_t)grp * nrows * NN;
-    for (int e = tid; e < nrows * NN; e += NT) sD[e] = src[e];
-    for (int e = tid; e < B * B; e += NT) sPairs[e] = pairs[e];
+    constexpr int EP = 16 / (int)sizeof(T), GS = (int)(Cfg::d_bytes(NN) / (int)sizeof(T));
+    const T* src = dtab + (size_t)grp * GS;
+    for (int e = tid; e < GS / EP; e += NT) cp_async<16>(sD + e * EP, src + e * EP, true);
+    for (int e = tid; e < B * B; e += NT) cp_async<8>(sPairs + e, pairs + e, true);
   }
   // one batch of coefficients: the rows arrive omega-blocked, [w / P][row][w % P],
   // one contiguous run per batch (from [row][omega], 32 bytes per row, the B = 15
@@ -302,14 +306,15 @@ int synth_real_launch(hp_plan* p, const c2<T>* Fp, T* f, cudaStream_t s) {
   const char* key = sizeof(T) == 8 ? "tf.sdn64" : "tf.sdn32";
   bool have = false;
   for (auto& kv : p->ws) if (kv.first == key) have = true;
-  const long long n = (long long)NG * p->nrows * NN, nd = (sizeof(T) * n + 15) / 16 * 16;
+  constexpr int gs = (int)(Cfg::d_bytes(NN) / (int)sizeof(T)), n = NG * gs;
+  constexpr size_t nd = sizeof(T) * (size_t)n;
   char* tab = (char*)p->ws_get(key, nd + sizeof(int2) * B * B, &st);
   if (st) return st;
   T* dtab = (T*)tab;
   int2* dpairs = (int2*)(tab + nd);
   if (!have) {
     k_sd_table<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
-        p->layout(), sizeof(T) == 8 ? (const T*)(const void*)p->wig64 : (const T*)(const void*)p->wig32, dtab, NN, NG);
+        p->layout(), sizeof(T) == 8 ? (const T*)(const void*)p->wig64 : (const T*)(const void*)p->wig32, dtab, NN, gs, NG);
     HP_CUDA_TRY(cudaGetLastError());
     k_node_pairs<B><<<(B * B + 127) / 128, 128, 0, s>>>(p->layout(), dpairs);
     HP_CUDA_TRY(cudaGetLastError());

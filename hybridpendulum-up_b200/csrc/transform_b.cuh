@@ -109,14 +109,14 @@ template <int B, bool CPLX> static const int2* pair_table(hp_plan* p, int* st, c
 }
 
 // (2l+1) d^l_mn at the first B nodes as [group][row][NN], group g holding the
-// nodes g NN .. g NN + NN-1 (zero past the last beta)
+// nodes g NN .. g NN + NN-1 (zero past the last beta); groups are gs values apart,
+// a multiple of 16 bytes
 template <typename T>
-__global__ void k_sd_table(RowLayout L, const T* __restrict__ wig, T* __restrict__ out, int NN, int ngroups) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= (long long)ngroups * L.nrows * NN) return;
-  const long long r = (t / NN) % L.nrows;
-  const int b = (int)(t / ((long long)NN * L.nrows)) * NN + (int)(t % NN);
-  out[t] = b < 2 * L.B ? (T)(2 * L.rows[r].x + 1) * wig[(size_t)b * L.nrows + r] : (T)0;
+__global__ void k_sd_table(RowLayout L, const T* __restrict__ wig, T* __restrict__ out, int NN, int gs, int ngroups) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= ngroups * gs) return;
+  const int g = t / gs, e = t - g * gs, r = e / NN, b = g * NN + e % NN;
+  out[t] = r < L.nrows && b < 2 * L.B ? (T)(2 * L.rows[r].x + 1) * wig[(size_t)b * L.nrows + r] : (T)0;
 }
 
 #include "synth.cuh"
