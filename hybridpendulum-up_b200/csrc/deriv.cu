@@ -474,7 +474,7 @@ __device__ __forceinline__ void plane_body(const RowLayout& L, const PlaneTile t
   const T d3 = HAS_P3 ? tp * (T)kappa_first(k3, N) : (T)0;
   T b1 = prm.b[0], b2 = prm.b[1], b3 = prm.b[2];
   T g1 = prm.g[0], g2 = prm.g[1], g3 = prm.g[2];
-  if constexpr (sizeof(T) == 4 && N > 30)   // registers to spare at two blocks per SM: keep them there
+  if constexpr (sizeof(T) == 4 && plane_minb<N, T, HAS_P3>() == 2)   // registers to spare at two blocks per SM
     asm volatile("" : "+f"(b1), "+f"(b2), "+f"(b3), "+f"(g1), "+f"(g2), "+f"(g3));
   for (int it = pr; it < tl.cnt * N * 2; it += npr) {   // both lanes of a pair hold the same item
     const int kind = it / (tl.cnt * N);
