@@ -85,10 +85,11 @@ __global__ void __launch_bounds__(128) k_axis3(RowLayout L, const c2<TIN>* __res
 // warp-uniform and reads shared memory only.  Per omega point the model part
 // of the weights folds into nu[n2] = -i sum_i D_i gs_i MR_i^1_{0 n2}, so
 //   G = noise F + sum_{n2} nu[n2] sum_{l1} w(l1, n2) F^{l1}_{m, n-n2}.
-// Bound by the shared-memory pipe: 9 source values per output, and the row's
-// weights and sources, which come as whole vectors from a table built with the
-// plan (one by one, with the sources recomputed by every block, the pass took
-// 0.49 ms at B = 15, 32^3, FP32 and 12.6 us at B = 8, 16 x 16; now 0.42 and 8.8).
+// Bound by issue slots in FP32 (86 % busy at B = 10, 32^3, the L1 and shared-memory
+// pipe 64 %): 9 source values per output, and the row's weights and sources, which
+// come as whole vectors from a table built with the plan (one by one, with the
+// sources recomputed by every block, the pass took 0.49 ms at B = 15, 32^3, FP32 and
+// 12.6 us at B = 8, 16 x 16; now 0.42 and 8.8).
 // The sources are offsets in the padding of the weights' rows: as nine more
 // values of two bytes they took shared memory from the tile (FP64 B = 22, 64 x 64:
 // 371 us, 294 now, 342 before there was a table; B = 12, 24^3: 159 and 147).
